@@ -247,11 +247,15 @@ def tensor_shapes(c):
 
 def tensors_of(case, seed):
     """The checkpoint: matrices N(0, 1 / fan-in), decays and step sizes spread so that some channels remember hundreds
-    of tokens and others a few, scores sharp enough that single keys count.  Matrices in the case's type, vectors in 32
-    bits."""
+    of tokens and others a few, scores sharp enough that single keys count.  A token's embedding leans towards the
+    directions of two experts and the routers follow them, so that, as in a trained model, most choices of experts are
+    clear (and none hangs on a rounding).  Matrices in the case's type, vectors in 32 bits."""
     g = torch.Generator(device=DEVICE).manual_seed(1000003 * int(seed) + 17)
     out = {}
     c = config_of(case)
+    routers = [layer["mlp"]["router"] for layer in c.get("layers", []) if layer["mlp"] and layer["mlp"]["kind"] == "moe"]
+    experts = routers[0]["experts"] + routers[0].get("identity", 0) if routers else 0
+    lean = torch.randn(max(experts, 1), c.get("width", 1), generator=g, device=DEVICE) / math.sqrt(c.get("width", 1))
     for name, shape in tensor_shapes(c).items():
         tail = name.split(".", 1)[1] if name[0] == "l" and name[1:2].isdigit() else name
 
@@ -280,12 +284,20 @@ def tensors_of(case, seed):
             t = normal(0.3, 1.0)
         elif tail == "mix.f.b":
             t = between(1.0, 5.0)
+        elif tail == "mlp.router":
+            t = lean + normal(0.3 / math.sqrt(shape[1]))
+        elif tail == "mlp.correction":
+            t = normal(0.02)
         elif len(shape) == 1:
             t = normal(0.3)
         elif "embed" in tail:
             t = normal()
+            if experts and name == "embed":
+                ids = torch.arange(shape[0], device=DEVICE)
+                first = ids % experts
+                t += 16.0 * (lean[first] + lean[(first + 1 + ids // experts % (experts - 1)) % experts])
         else:
-            wide = 3.0 if tail == "mlp.router" else 0.5 if tail.endswith((".o", "down", "o_proj.weight", "down_proj.weight")) else 1.0
+            wide = 0.5 if tail.endswith((".o", "down", "o_proj.weight", "down_proj.weight")) else 1.0
             t = normal(wide / math.sqrt(shape[1]))
         vector = len(shape) == 1 or tail.endswith((".conv", "A_log", "mlp.router"))
         out[name] = t.to(torch.bfloat16).float() if vector else t.to(TYPES[case["dtype"]])
@@ -484,10 +496,6 @@ def tolerance(case):
         return {"rel": 0.0, "differ": 0.05}           # (a sum in another order moves a boundary between two tokens)
     if case["dtype"] == "float32":
         return {"rel": 1e-5}                          # (1.5e-6 against 64 bits)
-    if case["model"].startswith(("ribozen", "zuzenex")):
-        # 0.01 to 0.036 over many rows, up to 0.1 over the eight of a replay's step: rounding sends some tokens to
-        # another expert
-        return {"rel": 0.4 if case["kind"] == "replay" else 0.14}
     return {"rel": 2.4e-2}                            # (0.004 to 0.006)
 
 
