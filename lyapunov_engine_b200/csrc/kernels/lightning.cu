@@ -32,11 +32,12 @@
 // (S from zero, no outputs) into scratch, the segments' starting states and
 // the request's new state row from those sums (element by element), and the
 // outputs of every segment from its starting state, all segments side by side.
-#include "common.cuh"
+#include "chunk_mma.cuh"
 
 namespace {
 
 using bf16 = __nv_bfloat16;
+using le::high_of, le::ldsm4, le::ldsm4_trans, le::low_of, le::mma, le::smem_addr, le::split_pair;
 
 // ---------------------------------------------------------------- scan
 constexpr int LS_THREADS = 256;
@@ -177,30 +178,6 @@ constexpr int SEGMENT = 256;
 constexpr int LC_COLS = 64;       // columns of S a block takes
 constexpr int LC_THREADS = 256;
 constexpr int LC_LDV = LC_COLS + 8;
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const bf16 *p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr(p)));
-}
-__device__ __forceinline__ void ldsm4_trans(uint32_t (&r)[4], const bf16 *p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr(p)));
-}
-__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// Two floats as two bfloat16 pairs whose sum keeps 16 bits of each.
-__device__ __forceinline__ void split_pair(float x, float y, uint32_t &high, uint32_t &low) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-  const __nv_bfloat162 l = __floats2bfloat162_rn(x - __low2float(h), y - __high2float(h));
-  high = *reinterpret_cast<const uint32_t *>(&h);
-  low = *reinterpret_cast<const uint32_t *>(&l);
-}
-__device__ __forceinline__ float low_of(uint32_t v) { return __uint_as_float(v << 16); }
-__device__ __forceinline__ float high_of(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 
 struct ChunkArgs {
   float *out; int64_t out_stride;

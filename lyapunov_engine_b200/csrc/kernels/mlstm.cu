@@ -46,6 +46,7 @@ struct MlstmArgs {
   const float *i_bias, *f_bias;
   float *state; int num_state_rows;
   const int32_t *state_slots, *cu_q;
+  const int32_t *requests;                        // the requests this launch takes, or null: all in order
   int heads, dim, vdim, rows_per_block;
   float cap, q_scale;
 };
@@ -62,7 +63,8 @@ mlstm_scan_kernel(MlstmArgs p) {
   float *s_gate = s_num + ML_TILE * ROWS;        // [6][TILE]: i, f, keep, take, floor, n . q
   __shared__ float s_m;                          // the running maximum between tiles
   le::let_successor_start();
-  const int b = blockIdx.z, head = blockIdx.y, e0 = blockIdx.x * ROWS;
+  const int b = p.requests != nullptr ? p.requests[blockIdx.z] : blockIdx.z;
+  const int head = blockIdx.y, e0 = blockIdx.x * ROWS;
   const int r = threadIdx.x / LANES, lane = threadIdx.x % LANES;
   const bool is_n = r == ROWS;                   // the group that carries n
   const int first = p.cu_q[b], q_len = p.cu_q[b + 1] - first;
@@ -271,13 +273,14 @@ int launch_mlstm_lanes(const MlstmArgs &p, int num_requests, cudaStream_t stream
 
 // out: float32 [T, heads * vdim].  rows (`dtype`): per token q [heads, dim] at q_col, k at k_col, v [heads, vdim] at
 // v_col and one pre-activation per head at i_col and at f_col.  state: float32 [num_state_rows, heads, vdim / R, R + 2,
-// dim] with R = le_mlstm_rows(dim, vdim).
+// dim] with R = le_mlstm_rows(dim, vdim).  requests: the indices of the num_requests requests to run, or null: requests
+// 0 .. num_requests - 1.
 LE_API int le_mlstm_rows(int dim, int vdim) { return dim >= 1 && vdim >= 1 ? ml_rows(dim, vdim) : 0; }
 
 LE_API int le_mlstm_scan(float *out, int64_t out_stride, const void *rows, int64_t row_stride, int q_col, int k_col, int v_col,
                          int i_col, int f_col, int dtype, const float *i_bias, const float *f_bias, float *state,
-                         int num_state_rows, const int32_t *state_slots, const int32_t *cu_q, int num_requests, int heads,
-                         int dim, int vdim, float cap, float q_scale, cudaStream_t stream) {
+                         int num_state_rows, const int32_t *state_slots, const int32_t *cu_q, const int32_t *requests,
+                         int num_requests, int heads, int dim, int vdim, float cap, float q_scale, cudaStream_t stream) {
   if (num_requests <= 0) return 0;
   if (heads < 1 || dim < 1 || vdim < 1 || heads > 65535 || num_requests > 65535)
     return le::invalid("le_mlstm_scan: %d heads of %d x %d for %d requests", heads, dim, vdim, num_requests);
@@ -286,7 +289,7 @@ LE_API int le_mlstm_scan(float *out, int64_t out_stride, const void *rows, int64
   p.out = out, p.out_stride = out_stride, p.qkv = rows, p.qkv_stride = row_stride;
   p.q_col = q_col, p.k_col = k_col, p.v_col = v_col, p.i_col = i_col, p.f_col = f_col;
   p.i_bias = i_bias, p.f_bias = f_bias, p.state = state, p.num_state_rows = num_state_rows;
-  p.state_slots = state_slots, p.cu_q = cu_q, p.heads = heads, p.dim = dim, p.vdim = vdim;
+  p.state_slots = state_slots, p.cu_q = cu_q, p.requests = requests, p.heads = heads, p.dim = dim, p.vdim = vdim;
   p.rows_per_block = ml_rows(dim, vdim), p.cap = cap, p.q_scale = q_scale;
   const int lanes = ml_lanes(dim);
 #define LE_ML(T)                                                                  \

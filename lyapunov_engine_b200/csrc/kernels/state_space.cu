@@ -43,6 +43,7 @@ struct SsmArgs {
   const float *dt_bias, *a_log, *d_skip;
   float *state; int num_state_rows;
   const int32_t *state_slots, *cu_q;
+  const int32_t *requests;                                 // the requests this launch takes, or null: all in order
   int rows, n_state, rows_per_head, rows_per_group, rows_per_block;
   float out_scale;
 };
@@ -59,7 +60,7 @@ ssm_scan_kernel(SsmArgs p) {
   float *s_y = s_dt + SSM_TILE * ROWS;         // [TILE][ROWS]
   float *s_dec = s_y + SSM_TILE * ROWS;        // [TILE][ROWS]: the decay of a row's head (one decay per head only)
   le::let_successor_start();
-  const int b = blockIdx.y;
+  const int b = p.requests != nullptr ? p.requests[blockIdx.y] : blockIdx.y;
   const int row0 = blockIdx.x * ROWS;
   const int r = threadIdx.x / LANES, lane = threadIdx.x % LANES;
   const int row = row0 + r;
@@ -308,13 +309,14 @@ static int ssm_rows_per_block(int n_state, int rows, int rows_per_group, int spr
 // [T, rows or heads], z [T, rows] or null: all of type `dtype`; out [T, rows] of type `out_dtype`.  per_row 1: dt,
 // dt_bias and d_skip have one entry per row and a_log is [rows, n_state]; 0: one per head of rows_per_head rows.
 // state: float32 [num_state_rows, rows, n_state]; request b (tokens cu_q[b] .. cu_q[b + 1]) owns row state_slots[b];
-// num_tokens: the step's tokens in all (it only chooses the launch's shape).
+// requests: the indices of the num_requests requests to run, or null: requests 0 .. num_requests - 1.  num_tokens: their
+// tokens in all (it only chooses the launch's shape).
 LE_API int le_ssm_scan(void *out, int out_dtype, int64_t out_stride, const void *x, int64_t x_stride, const void *bc,
                        int64_t bc_stride, int b_col, int c_col, const void *dt, int64_t dt_stride, const void *z,
                        int64_t z_stride, int dtype, const float *dt_bias, const float *a_log, const float *d_skip,
-                       float *state, int num_state_rows, const int32_t *state_slots, const int32_t *cu_q, int num_requests,
-                       int num_tokens, int rows, int n_state, int rows_per_head, int rows_per_group, int per_row,
-                       float out_scale, cudaStream_t stream) {
+                       float *state, int num_state_rows, const int32_t *state_slots, const int32_t *cu_q,
+                       const int32_t *requests, int num_requests, int num_tokens, int rows, int n_state, int rows_per_head,
+                       int rows_per_group, int per_row, float out_scale, cudaStream_t stream) {
   if (num_requests <= 0 || rows <= 0) return 0;
   if (num_requests > 65535) return le::invalid("le_ssm_scan: too many requests for one launch");
   if (n_state < 1 || rows_per_head < 1 || rows_per_group < 1 || rows % rows_per_group || rows_per_group % rows_per_head)
@@ -323,8 +325,8 @@ LE_API int le_ssm_scan(void *out, int out_dtype, int64_t out_stride, const void 
   p.x = x, p.x_stride = x_stride, p.bc = bc, p.bc_stride = bc_stride, p.b_col = b_col, p.c_col = c_col;
   p.dt = dt, p.dt_stride = dt_stride, p.z = z, p.z_stride = z_stride, p.out = out, p.out_stride = out_stride;
   p.dt_bias = dt_bias, p.a_log = a_log, p.d_skip = d_skip, p.state = state, p.num_state_rows = num_state_rows;
-  p.state_slots = state_slots, p.cu_q = cu_q, p.rows = rows, p.n_state = n_state, p.rows_per_head = rows_per_head;
-  p.rows_per_group = rows_per_group, p.out_scale = out_scale;
+  p.state_slots = state_slots, p.cu_q = cu_q, p.requests = requests, p.rows = rows, p.n_state = n_state;
+  p.rows_per_head = rows_per_head, p.rows_per_group = rows_per_group, p.out_scale = out_scale;
   const int spread = per_row && num_tokens > num_requests;
   p.rows_per_block = ssm_rows_per_block(n_state, rows, rows_per_group, spread, num_requests);
   const int lanes = ssm_lanes(n_state, spread);

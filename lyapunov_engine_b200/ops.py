@@ -111,8 +111,15 @@ _CORE_SIGNATURES = {
     "le_stream_entry": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p],
     "le_sigmoid_gate": [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_float, c_void_p],
     "le_ssm_scan": [c_void_p, c_int, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_void_p, c_int64, c_void_p,
-                    c_int64, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                    c_int, c_int, c_int, c_float, c_void_p],
+                    c_int64, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                    c_int, c_int, c_int, c_int, c_int, c_float, c_void_p],
+    "le_decay_segment": [],
+    "le_duality_chunks": [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_void_p, c_int64, c_void_p,
+                          c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
+                          c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p],
+    "le_memory_chunks": [c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
+                         c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
+                         c_float, c_void_p, c_void_p, c_void_p],
     "le_activate": [c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_void_p],
     "le_lightning_segment": [],
     "le_lightning_scan": [c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
@@ -121,7 +128,7 @@ _CORE_SIGNATURES = {
                             c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "le_mlstm_rows": [c_int, c_int],
     "le_mlstm_scan": [c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                      c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p],
+                      c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p],
     "le_rope_qknorm_store": [c_void_p, c_int64, c_int, c_void_p, c_void_p, c_void_p, c_float, c_int, c_int, c_void_p, c_int,
                              c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                              c_int, c_int, c_int, c_void_p, c_void_p],
@@ -1636,7 +1643,7 @@ SSM_MAX_STATE = 512
 
 
 def ssm_scan(out, x, bc, b_col: int, c_col: int, dt, z, dt_bias, a_log, d_skip, state, state_slots, cu_q, num_requests: int,
-             n_state: int, rows_per_head: int, rows_per_group: int, per_row: bool, out_scale: float = 1.0) -> None:
+             n_state: int, rows_per_head: int, rows_per_group: int, per_row: bool, out_scale: float = 1.0, requests=None) -> None:
     """A diagonal state-space recurrence over the step's tokens, request by
     request, from each request's state row and back into it.  Per row r
     (channel) with N = ``n_state`` numbers of state, per token:
@@ -1648,8 +1655,9 @@ def ssm_scan(out, x, bc, b_col: int, c_col: int, dt, z, dt_bias, a_log, d_skip, 
     ``b_col`` and C at ``c_col``; the rows of a group (``rows_per_group``
     consecutive ones) share them.  ``x``, ``bc``, ``dt``, ``z`` are column
     ranges of rows in the activations' type; ``out`` that type or float32;
-    ``state`` float32 [state rows, rows, N]."""
-    _need_cuda(out, x, bc, dt, z, dt_bias, a_log, d_skip, state, state_slots, cu_q)
+    ``state`` float32 [state rows, rows, N].  ``requests``: int32 indices of
+    the ``num_requests`` requests to run (None: the first ones)."""
+    _need_cuda(out, x, bc, dt, z, dt_bias, a_log, d_skip, state, state_slots, cu_q, requests)
     T, rows = x.shape
     assert out.shape == (T, rows) and out.stride(1) == 1 and x.stride(1) == 1 and bc.stride(1) == 1 and dt.stride(1) == 1
     assert x.dtype == bc.dtype == dt.dtype and (z is None or (z.dtype == x.dtype and z.stride(1) == 1 and z.shape == x.shape))
@@ -1661,20 +1669,67 @@ def ssm_scan(out, x, bc, b_col: int, c_col: int, dt, z, dt_bias, a_log, d_skip, 
     _check(core().le_ssm_scan(_ptr(out), dtype_code(out.dtype), out.stride(0), _ptr(x), x.stride(0), _ptr(bc), bc.stride(0),
                               int(b_col), int(c_col), _ptr(dt), dt.stride(0), _ptr(z), z.stride(0) if z is not None else 0,
                               dtype_code(x.dtype), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), state.shape[0],
-                              _ptr(state_slots), _ptr(cu_q), int(num_requests), T, rows, int(n_state), int(rows_per_head),
+                              _ptr(state_slots), _ptr(cu_q), _ptr(requests), int(num_requests),
+                              T if requests is None else int(num_requests), rows, int(n_state), int(rows_per_head),
                               int(rows_per_group), 1 if per_row else 0, float(out_scale), _stream()), "le_ssm_scan")
+
+
+DECAY_CHUNK_MAX_DIM = 128          # entries of a head's keys that the forms over chunks take
+_segment_sizes: dict[str, int] = {}
+
+
+def decay_segment() -> int:
+    """Tokens per segment of duality_chunks() and memory_chunks()."""
+    if "decay" not in _segment_sizes:
+        _segment_sizes["decay"] = int(core().le_decay_segment())
+    return _segment_sizes["decay"]
+
+
+def decay_work_floats(num_segments: int, num_tokens: int, heads: int, dim: int) -> int:
+    """Floats of ``work`` that duality_chunks() and memory_chunks() fill (decays and weights per head and token, decays
+    per head and segment, the matrix memory's vectors n)."""
+    return 4 * heads * num_tokens + num_segments * heads * (1 + dim)
+
+
+def duality_chunks(out, x, bc, b_col: int, c_col: int, dt, z, dt_bias, a_log, d_skip, state, state_slots, cu_q, tile_request,
+                   tile_q0, num_segments: int, n_state: int, rows_per_head: int, rows_per_group: int, work, scratch,
+                   out_scale: float = 1.0) -> None:
+    """ssm_scan() with one decay per head, over chunks on the tensor cores, for
+    the requests whose segments (decay_segment() tokens each, a request's in
+    their order) the first ``num_segments`` entries of the tile lists name.
+    Rows bfloat16, ``out`` float32, at most DECAY_CHUNK_MAX_DIM numbers of
+    state per channel.  ``work``: decay_work_floats() floats; ``scratch``:
+    float32 [num_segments, rows, n_state] where a request has several
+    segments, else None."""
+    _need_cuda(out, x, bc, dt, z, dt_bias, a_log, d_skip, state, state_slots, cu_q, tile_request, tile_q0, work, scratch)
+    T, rows = x.shape
+    heads = rows // rows_per_head
+    assert out.dtype == torch.float32 and out.shape == (T, rows) and out.stride(1) == 1 and x.stride(1) == 1 and bc.stride(1) == 1
+    assert x.dtype == bc.dtype == dt.dtype == torch.bfloat16 and dt.stride(1) == 1 and dt.shape[1] >= heads
+    assert z is None or (z.dtype == x.dtype and z.stride(1) == 1 and z.shape == x.shape)
+    assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (rows, n_state)
+    assert n_state <= DECAY_CHUNK_MAX_DIM and rows_per_group % rows_per_head == 0
+    assert dt_bias.dtype == a_log.dtype == torch.float32 and dt_bias.numel() == a_log.numel() == heads
+    assert d_skip is None or (d_skip.dtype == torch.float32 and d_skip.numel() == heads)
+    assert work.dtype == torch.float32 and work.is_contiguous() and work.numel() >= decay_work_floats(num_segments, T, heads, n_state)
+    assert scratch is None or (scratch.dtype == torch.float32 and scratch.is_contiguous()
+                               and scratch.numel() >= num_segments * rows * n_state)
+    _check(core().le_duality_chunks(_ptr(out), out.stride(0), _ptr(x), x.stride(0), _ptr(bc), bc.stride(0), int(b_col), int(c_col),
+                                    _ptr(dt), dt.stride(0), _ptr(z), z.stride(0) if z is not None else 0, _ptr(dt_bias),
+                                    _ptr(a_log), _ptr(d_skip), _ptr(state), state.shape[0], _ptr(state_slots), _ptr(cu_q),
+                                    _ptr(tile_request), _ptr(tile_q0), int(num_segments), T, heads, int(rows_per_head),
+                                    int(n_state), int(rows_per_group) // int(rows_per_head), float(out_scale), _ptr(work),
+                                    _ptr(scratch), _stream()), "le_duality_chunks", launches=2 if scratch is None else 4)
 
 
 LIGHTNING_MAX_DIM = 512
 LIGHTNING_CHUNK_MAX_DIM = 128      # of the form over chunks
-_lightning_sizes: dict[str, int] = {}
-
 
 def lightning_segment() -> int:
     """Tokens per segment of lightning_chunks()."""
-    if "segment" not in _lightning_sizes:
-        _lightning_sizes["segment"] = int(core().le_lightning_segment())
-    return _lightning_sizes["segment"]
+    if "lightning" not in _segment_sizes:
+        _segment_sizes["lightning"] = int(core().le_lightning_segment())
+    return _segment_sizes["lightning"]
 
 
 def lightning_tables(decay, device):
@@ -1744,9 +1799,17 @@ def mlstm_state_shape(heads: int, dim: int, vdim: int) -> tuple:
     return (heads, vdim // r, r + 2, dim)
 
 
+def _mlstm_checks(out, rows, i_bias, f_bias, state, heads, dim, vdim) -> None:
+    assert out.dtype == torch.float32 and out.shape == (rows.shape[0], heads * vdim) and out.stride(1) == 1 and rows.stride(1) == 1
+    assert i_bias.dtype == torch.float32 and f_bias.dtype == torch.float32 and i_bias.numel() == heads and f_bias.numel() == heads
+    assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == mlstm_state_shape(heads, dim, vdim)
+
+
 def mlstm_scan(out, rows, q_col: int, k_col: int, v_col: int, i_col: int, f_col: int, i_bias, f_bias, state, state_slots, cu_q,
-               num_requests: int, heads: int, dim: int, vdim: int, cap: float, q_scale: float) -> None:
-    """The mLSTM's matrix memory over the step's tokens, request by request.
+               num_requests: int, heads: int, dim: int, vdim: int, cap: float, q_scale: float, requests=None) -> None:
+    """The mLSTM's matrix memory over the step's tokens, request by request
+    (``requests``: int32 indices of the ``num_requests`` ones to run; None:
+    the first ones).
     ``rows``: per token q, k [heads, dim], v [heads, vdim] and one gate
     pre-activation per head for the input and the forget gate, at the given
     columns.  With i = cap tanh((a_i + b_i) / cap), f = logsigmoid(cap
@@ -1755,15 +1818,33 @@ def mlstm_scan(out, rows, q_col: int, k_col: int, v_col: int, i_col: int, f_col:
         out = S^T (q * q_scale) / (max(|n . q * q_scale|, e^(-m')) + 1e-6)
     ``out`` float32 [T, heads * vdim]; ``state`` float32 [state rows,
     *mlstm_state_shape()]."""
-    _need_cuda(out, rows, i_bias, f_bias, state, state_slots, cu_q)
-    T = rows.shape[0]
-    assert out.dtype == torch.float32 and out.shape == (T, heads * vdim) and out.stride(1) == 1 and rows.stride(1) == 1
-    assert i_bias.dtype == torch.float32 and f_bias.dtype == torch.float32 and i_bias.numel() == heads and f_bias.numel() == heads
-    assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == mlstm_state_shape(heads, dim, vdim)
+    _need_cuda(out, rows, i_bias, f_bias, state, state_slots, cu_q, requests)
+    _mlstm_checks(out, rows, i_bias, f_bias, state, heads, dim, vdim)
     _check(core().le_mlstm_scan(_ptr(out), out.stride(0), _ptr(rows), rows.stride(0), int(q_col), int(k_col), int(v_col),
                                 int(i_col), int(f_col), dtype_code(rows.dtype), _ptr(i_bias), _ptr(f_bias), _ptr(state),
-                                state.shape[0], _ptr(state_slots), _ptr(cu_q), int(num_requests), int(heads), int(dim), int(vdim),
-                                float(cap), float(q_scale), _stream()), "le_mlstm_scan")
+                                state.shape[0], _ptr(state_slots), _ptr(cu_q), _ptr(requests), int(num_requests), int(heads),
+                                int(dim), int(vdim), float(cap), float(q_scale), _stream()), "le_mlstm_scan")
+
+
+def memory_chunks(out, rows, q_col: int, k_col: int, v_col: int, i_col: int, f_col: int, i_bias, f_bias, state, state_slots, cu_q,
+                  tile_request, tile_q0, num_segments: int, heads: int, dim: int, vdim: int, cap: float, q_scale: float, work,
+                  scratch) -> None:
+    """mlstm_scan() over chunks on the tensor cores (bfloat16 rows, heads of at
+    most DECAY_CHUNK_MAX_DIM entries); the lists and ``work`` as for
+    duality_chunks(), ``scratch`` float32 [num_segments, heads, vdim + 1,
+    dim] where a request has several segments, else None."""
+    _need_cuda(out, rows, i_bias, f_bias, state, state_slots, cu_q, tile_request, tile_q0, work, scratch)
+    _mlstm_checks(out, rows, i_bias, f_bias, state, heads, dim, vdim)
+    T = rows.shape[0]
+    assert rows.dtype == torch.bfloat16 and dim <= DECAY_CHUNK_MAX_DIM
+    assert work.dtype == torch.float32 and work.is_contiguous() and work.numel() >= decay_work_floats(num_segments, T, heads, dim)
+    assert scratch is None or (scratch.dtype == torch.float32 and scratch.is_contiguous()
+                               and scratch.numel() >= num_segments * heads * (vdim + 1) * dim)
+    _check(core().le_memory_chunks(_ptr(out), out.stride(0), _ptr(rows), rows.stride(0), int(q_col), int(k_col), int(v_col),
+                                   int(i_col), int(f_col), _ptr(i_bias), _ptr(f_bias), _ptr(state), state.shape[0],
+                                   _ptr(state_slots), _ptr(cu_q), _ptr(tile_request), _ptr(tile_q0), int(num_segments), T,
+                                   int(heads), int(dim), int(vdim), mlstm_rows(dim, vdim), float(cap), float(q_scale), _ptr(work),
+                                   _ptr(scratch), _stream()), "le_memory_chunks", launches=2 if scratch is None else 4)
 
 
 def rope_qknorm_store(rows, bias, w_q, w_k, eps, q_count, k_count, rates, rot, magnitude, k_cache, v_cache, positions,

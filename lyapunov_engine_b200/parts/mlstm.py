@@ -12,7 +12,9 @@ With x the mixer's input, H heads, d the query/key size and e the value size:
 
 S, n and m are carried from token to token in 32 bits, per request and head
 (``state_need``).  One product makes all six projections; the recurrence and
-the gated norm are a kernel each (ops.mlstm_scan, ops.head_norm_gate).  The
+the gated norm are a kernel each (ops.mlstm_scan, ops.head_norm_gate); requests
+that bring several tokens in bfloat16 go over chunks on the tensor cores
+(ops.memory_chunks).  The
 gates, the recurrence and the norm are 32-bit.
 """
 from __future__ import annotations
@@ -21,6 +23,8 @@ import torch
 
 from .. import ops
 from .base import Mixer, StateNeed, TensorDecl, register_mixer
+
+SEGMENT = 256      # tokens of a request that a block of the chunked form takes
 
 
 @register_mixer("matrix_memory")
@@ -48,6 +52,9 @@ class MatrixMemoryMixer(Mixer):
     def state_need(self):
         return StateNeed(ops.mlstm_state_shape(self.num_heads, self.head_dim, self.value_dim), torch.float32)
 
+    def tile_sizes(self):
+        return [SEGMENT]
+
     def tensors(self):
         q, k, v, g, i, f = self.names
         W, H, d, e = self.hidden_size, self.num_heads, self.head_dim, self.value_dim
@@ -68,6 +75,8 @@ class MatrixMemoryMixer(Mixer):
         self.f_bias = get(self.names[5] + self.bias_suffix).contiguous()
         self.norm_weight = get(self.norm_name).contiguous()
         self.w_o = get(self.o_name)
+        if ops.decay_segment() != SEGMENT:
+            raise RuntimeError(f"the kernels' segments have {ops.decay_segment()} tokens, the mixer lists {SEGMENT}")
         self.runtime = runtime
 
     def inner_width(self) -> int:
@@ -88,8 +97,21 @@ class MatrixMemoryMixer(Mixer):
         proj = ws.get("mlstm_proj", (T, self.width), rt.dtype)
         ops.linear(proj, x, self.w_in, ctx.status)
         o = ws.get("mlstm_out", (T, H * e), torch.float32)
-        ops.mlstm_scan(o, proj, self.q_col, self.k_col, self.v_col, self.i_col, self.f_col, self.i_bias, self.f_bias,
-                       cache.state, ctx.state_slots, ctx.cu_q, ctx.num_requests, H, d, e, self.gate_cap, d ** -0.5)
+        rows = (o, proj, self.q_col, self.k_col, self.v_col, self.i_col, self.f_col, self.i_bias, self.f_bias, cache.state,
+                ctx.state_slots, ctx.cu_q)
+        sizes = (H, d, e, self.gate_cap, d ** -0.5)
+        request, q0, _, segments = ctx.tiles[SEGMENT]
+        if segments and rt.dtype == torch.bfloat16 and d <= ops.DECAY_CHUNK_MAX_DIM:
+            # (a step in which no request has a second segment goes from state row to state row)
+            scratch = None
+            if segments > ctx.num_requests - ctx.num_decode:
+                scratch = ws.get("mlstm_scratch", (segments, H, e + 1, d), torch.float32)
+            work = ws.get("mlstm_work", (ops.decay_work_floats(segments, T, H, d),), torch.float32)
+            ops.memory_chunks(*rows, request, q0, segments, *sizes, work, scratch)
+            if ctx.num_decode:
+                ops.mlstm_scan(*rows, ctx.num_decode, *sizes, requests=ctx.decode_requests)
+        else:
+            ops.mlstm_scan(*rows, ctx.num_requests, *sizes)
         if out is None:
             out = ws.get("mlstm_gated", (T, H * e), rt.dtype)
         ops.head_norm_gate(out, o, proj[:, self.gate_col:self.gate_col + H * e], self.norm_weight, self.norm_eps, H, e,

@@ -20,7 +20,8 @@ G)), inner = H * P:
     y <- y * silu(z);  W_o
 
 Both recurrences run in one kernel (ops.ssm_scan), with the gate in its
-epilogue; the convolution is the package's short convolution with a bias and
+epilogue; requests that bring several tokens in bfloat16 go through the duality
+over chunks on the tensor cores instead (ops.duality_chunks).  The convolution is the package's short convolution with a bias and
 silu; the last taps - 1 inputs of the convolution are state of the request too
 (``extra_state_needs``).  Step sizes, decays, the recurrence and the norm are
 32-bit.
@@ -31,6 +32,8 @@ import torch
 
 from .. import ops
 from .base import Mixer, StateNeed, TensorDecl, register_mixer
+
+SEGMENT = 256      # tokens of a request that a block of the duality's chunked form takes
 
 
 def _conv(out, rows, channels, mixer, ctx, cache):
@@ -88,7 +91,7 @@ class StateSpaceDualityMixer(Mixer):
         return {"mixer_taps": StateNeed((self.taps - 1, self.channels), torch.float32)}
 
     def tile_sizes(self):
-        return [ops.SHORT_CONV_TILE]
+        return [ops.SHORT_CONV_TILE, SEGMENT]
 
     def tensors(self):
         W, H, GN = self.hidden_size, self.num_heads, self.groups * self.state_dim
@@ -111,6 +114,8 @@ class StateSpaceDualityMixer(Mixer):
         self.dt_bias, self.a_log, self.d_skip = get(self.dt_bias_name), get(self.a_log_name), get(self.d_name)
         self.norm_weight = get(self.norm_name)
         self.w_o = get(self.o_name)
+        if ops.decay_segment() != SEGMENT:
+            raise RuntimeError(f"the kernels' segments have {ops.decay_segment()} tokens, the mixer lists {SEGMENT}")
         self.runtime = runtime
 
     def inner_width(self) -> int:
@@ -133,9 +138,21 @@ class StateSpaceDualityMixer(Mixer):
         conv = ws.get("ssd_conv", (T, self.channels), rt.dtype)
         _conv(conv, proj, self.channels, self, ctx, cache)
         y = ws.get("ssd_y", (T, inner), torch.float32)
-        ops.ssm_scan(y, conv[:, :inner], conv, inner, inner + self.groups * N, proj[:, self.dt_col:self.dt_col + H],
-                     proj[:, self.z_col:self.z_col + inner], self.dt_bias, self.a_log, self.d_skip, cache.state, ctx.state_slots,
-                     ctx.cu_q, ctx.num_requests, N, self.value_dim, (H // self.groups) * self.value_dim, per_row=False)
+        rows = (y, conv[:, :inner], conv, inner, inner + self.groups * N, proj[:, self.dt_col:self.dt_col + H],
+                proj[:, self.z_col:self.z_col + inner], self.dt_bias, self.a_log, self.d_skip, cache.state, ctx.state_slots, ctx.cu_q)
+        sizes = (N, self.value_dim, (H // self.groups) * self.value_dim)
+        request, q0, _, segments = ctx.tiles[SEGMENT]
+        if segments and rt.dtype == torch.bfloat16 and N <= ops.DECAY_CHUNK_MAX_DIM:
+            # (a step in which no request has a second segment goes from state row to state row)
+            scratch = None
+            if segments > ctx.num_requests - ctx.num_decode:
+                scratch = ws.get("ssd_scratch", (segments, inner, N), torch.float32)
+            work = ws.get("ssd_work", (ops.decay_work_floats(segments, T, H, N),), torch.float32)
+            ops.duality_chunks(*rows, request, q0, segments, *sizes, work, scratch)
+            if ctx.num_decode:
+                ops.ssm_scan(*rows, ctx.num_decode, *sizes, per_row=False, requests=ctx.decode_requests)
+        else:
+            ops.ssm_scan(*rows, ctx.num_requests, *sizes, per_row=False)
         normed = ws.get("ssd_normed", (T, inner), rt.dtype)
         ops.rmsnorm(normed, y, None, self.norm_weight, self.norm_eps, groups=self.norm_groups)
         return normed
