@@ -20,9 +20,10 @@
 // registers.  The request's tokens pass in tiles of TILE through shared memory
 // (B and C of the group, x, step sizes and gates of the block's rows); within
 // a tile the threads run without meeting, the tile's outputs leave together.
-// One launch serves every cut of the work: a request brings its next q_len
-// tokens, 1 for a decoded token.  Requests without a state row (slot < 0,
-// padding of a fixed-shape step) are skipped; their output rows are zeroed.
+// One launch of the scan serves every cut of the work: a request brings its next q_len
+// tokens, 1 for a decoded token (prompts with a decay per row and state have a
+// form of their own below).  Requests without a state row (slot < 0, padding of
+// a fixed-shape step) are skipped; their output rows are zeroed.
 #include "common.cuh"
 
 namespace {
@@ -243,6 +244,243 @@ ssm_scan_kernel(SsmArgs p) {
   }
 }
 
+// ---------------------------------------------------------------- segments of tokens side by side
+// The form with a decay per row and state for requests that bring several tokens (bfloat16 rows, one group, up to
+// SEG_STATE numbers of state per row).  Walked token by token a prompt is a chain of dependent steps and a request's
+// rows are all the threads there are (2,048 rows of 16 numbers, 2,048 tokens: 601 us, now 164 us; error against 64 bits
+// 1.62e-7, now 1.47e-7).  Here segments of SEG_TOKENS tokens run side by side, a thread per row with the row's whole
+// state in registers:
+//   selective_segment_kernel<SUMS>   each segment from a zero state: the state it ends in, and the sum of its step sizes
+//                                    (a request's last segment is left out: nothing follows it);
+//   selective_starts_kernel          down the segments of a request, per number of state: the state each starts from,
+//                                    S <- exp(A sum) S + its own end (decays of one rate multiply to one exponential);
+//   selective_segment_kernel<!SUMS>  each segment from its state, with the outputs; the last one leaves the request's.
+// What bounds it: the decays' exponentials (one per token and number of state, in both passes); they are made two at
+// a time in packed multiply-adds, and a thread's 16 chains cover one another's latencies.  64 tokens a segment: with
+// 128 a prompt of 2,048 tokens is 256 blocks of four warps, fewer than two for every multiprocessor.
+constexpr int SEG_TOKENS = 64;
+constexpr int SEG_STATE = 16;
+constexpr int SEG_THREADS = 128;
+constexpr int SEG_AHEAD = 4;       // tokens whose x, step size and gate are asked for before they are used
+
+struct SegArgs {
+  const int32_t *tile_request, *tile_q0;     // the segments: their requests, their first tokens within them
+  float *scratch;                            // [segments, rows, N]: the segments' own ends, then the states they start from
+  float *sums;                               // [segments, rows]: their step sizes added up
+};
+
+// e^x of two numbers <= 0: le::exp_unbiased's reduction and polynomial in packed operations.
+__device__ __forceinline__ float2 exp_pair(float2 x) {
+  const float2 magic = make_float2(12582912.0f, 12582912.0f);          // 1.5 * 2^23: a sum with it is rounded to whole numbers
+  x.x = fmaxf(x.x, -87.0f), x.y = fmaxf(x.y, -87.0f);
+  const float2 t = __ffma2_rn(x, make_float2(1.44269504f, 1.44269504f), magic);
+  const float2 k = __fadd2_rn(t, make_float2(-12582912.0f, -12582912.0f));
+  float2 r = __ffma2_rn(k, make_float2(-0.693145752f, -0.693145752f), x);
+  r = __ffma2_rn(k, make_float2(-1.42860677e-06f, -1.42860677e-06f), r);
+  float2 p = make_float2(1.9875691500e-4f, 1.9875691500e-4f);
+  p = __ffma2_rn(p, r, make_float2(1.3981999507e-3f, 1.3981999507e-3f));
+  p = __ffma2_rn(p, r, make_float2(8.3334519073e-3f, 8.3334519073e-3f));
+  p = __ffma2_rn(p, r, make_float2(4.1665795894e-2f, 4.1665795894e-2f));
+  p = __ffma2_rn(p, r, make_float2(1.6666665459e-1f, 1.6666665459e-1f));
+  p = __ffma2_rn(p, r, make_float2(5.0000001201e-1f, 5.0000001201e-1f));
+  const float2 e = __fadd2_rn(__ffma2_rn(__fmul2_rn(r, r), p, r), make_float2(1.0f, 1.0f));
+  // (the low bits of t are k: into e's exponent)
+  return make_float2(__int_as_float(__float_as_int(e.x) + (__float_as_int(t.x) << 23)),
+                     __int_as_float(__float_as_int(e.y) + (__float_as_int(t.y) << 23)));
+}
+
+template <typename TO, bool SUMS>
+__global__ void __launch_bounds__(SEG_THREADS)
+selective_segment_kernel(SsmArgs p, SegArgs s) {
+  using bf16 = __nv_bfloat16;
+  __shared__ __align__(16) float s_b[SEG_TOKENS][SEG_STATE];
+  __shared__ __align__(16) float s_c[SUMS ? 1 : SEG_TOKENS][SEG_STATE];
+  le::let_successor_start();
+  const int N = p.n_state;
+  const int seg = blockIdx.y;
+  const int row = blockIdx.x * SEG_THREADS + threadIdx.x;
+  const bool active = row < p.rows;
+  const int b = s.tile_request[seg], q0 = s.tile_q0[seg];
+  const int left = p.cu_q[b + 1] - p.cu_q[b] - q0;
+  const int tokens = min(SEG_TOKENS, left);
+  const bool last = left <= SEG_TOKENS;
+  if (SUMS && last) return;
+  const int64_t first = static_cast<int64_t>(p.cu_q[b]) + q0;
+  const int slot = p.state_slots[b];
+  const bool has_state = slot >= 0 && slot < p.num_state_rows;
+
+  float2 a[SEG_STATE / 2];                       // (zero behind the row's N numbers: their state stays zero)
+  float bias = 0.0f, d_skip = 0.0f;
+#pragma unroll
+  for (int n = 0; n < SEG_STATE / 2; ++n) a[n] = make_float2(0.0f, 0.0f);
+  if (active) {
+    bias = p.dt_bias[row];
+    d_skip = p.d_skip != nullptr ? p.d_skip[row] : 0.0f;
+    const float *rates = p.a_log + static_cast<int64_t>(row) * N;
+#pragma unroll
+    for (int n = 0; n < SEG_STATE; n += 2) {
+      if (n < N) a[n / 2].x = -expf(rates[n]);
+      if (n + 1 < N) a[n / 2].y = -expf(rates[n + 1]);
+    }
+  }
+  le::wait_for_predecessor();
+
+  const bf16 *bcs = static_cast<const bf16 *>(p.bc) + first * p.bc_stride;
+  constexpr int PIECE = 8;
+  const bool pieces = N % PIECE == 0 && p.b_col % PIECE == 0 && p.c_col % PIECE == 0 && p.bc_stride % PIECE == 0 &&
+                      (reinterpret_cast<uintptr_t>(p.bc) & 15) == 0;
+  if (pieces) {
+    for (int i = threadIdx.x; i < tokens * (SEG_STATE / PIECE); i += SEG_THREADS) {
+      const int t = i / (SEG_STATE / PIECE), n = i % (SEG_STATE / PIECE) * PIECE;
+      float bv[PIECE] = {}, cv[PIECE] = {};
+      if (n < N) {
+        le::load_piece16<bf16>(bv, bcs + t * p.bc_stride + p.b_col + n);
+        if constexpr (!SUMS) le::load_piece16<bf16>(cv, bcs + t * p.bc_stride + p.c_col + n);
+      }
+#pragma unroll
+      for (int v = 0; v < PIECE; v += 4) {
+        *reinterpret_cast<float4 *>(&s_b[t][n + v]) = make_float4(bv[v], bv[v + 1], bv[v + 2], bv[v + 3]);
+        if constexpr (!SUMS) *reinterpret_cast<float4 *>(&s_c[t][n + v]) = make_float4(cv[v], cv[v + 1], cv[v + 2], cv[v + 3]);
+      }
+    }
+  } else {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < tokens * SEG_STATE; i += SEG_THREADS) {
+      const int t = i / SEG_STATE, n = i % SEG_STATE;
+      s_b[t][n] = n < N ? __bfloat162float(bcs[t * p.bc_stride + p.b_col + n]) : 0.0f;
+      if constexpr (!SUMS) s_c[t][n] = n < N ? __bfloat162float(bcs[t * p.bc_stride + p.c_col + n]) : 0.0f;
+    }
+  }
+
+  float2 S[SEG_STATE / 2];
+#pragma unroll
+  for (int n = 0; n < SEG_STATE / 2; ++n) S[n] = make_float2(0.0f, 0.0f);
+  float *kept = has_state && active ? p.state + (static_cast<int64_t>(slot) * p.rows + row) * N : nullptr;
+  float *piece = s.scratch != nullptr && active ? s.scratch + (static_cast<int64_t>(seg) * p.rows + row) * N : nullptr;
+  if constexpr (!SUMS) {
+    const float *from = piece != nullptr ? piece : kept;
+    if (from != nullptr) {
+#pragma unroll
+      for (int n = 0; n < SEG_STATE; n += 2) {
+        if (n < N) S[n / 2].x = from[n];
+        if (n + 1 < N) S[n / 2].y = from[n + 1];
+      }
+    }
+  }
+  const bf16 *xs = static_cast<const bf16 *>(p.x) + first * p.x_stride + row;
+  const bf16 *dts = static_cast<const bf16 *>(p.dt) + first * p.dt_stride + row;
+  const bf16 *zs = p.z != nullptr ? static_cast<const bf16 *>(p.z) + first * p.z_stride + row : nullptr;
+  TO *outs = static_cast<TO *>(p.out) + first * p.out_stride + row;
+  __syncthreads();
+  if (!active) return;
+  if (!SUMS && !has_state) {
+    for (int t = 0; t < tokens; ++t) outs[t * p.out_stride] = le::from_f32<TO>(0.0f);
+    return;
+  }
+  bf16 x_next[SEG_AHEAD], dt_next[SEG_AHEAD], z_next[SEG_AHEAD];
+  const bf16 none = __float2bfloat16_rn(0.0f);
+  auto ask = [&](int t0) {
+#pragma unroll
+    for (int u = 0; u < SEG_AHEAD; ++u) {
+      const int t = t0 + u;
+      x_next[u] = dt_next[u] = z_next[u] = none;
+      if (t < tokens) {
+        x_next[u] = xs[t * p.x_stride];
+        dt_next[u] = dts[t * p.dt_stride];
+        if (!SUMS && zs != nullptr) z_next[u] = zs[t * p.z_stride];
+      }
+    }
+  };
+  ask(0);
+  float sum = 0.0f;
+  for (int t0 = 0; t0 < tokens; t0 += SEG_AHEAD) {
+    float xv[SEG_AHEAD], step[SEG_AHEAD], g[SEG_AHEAD];
+#pragma unroll
+    for (int u = 0; u < SEG_AHEAD; ++u) {
+      xv[u] = __bfloat162float(x_next[u]);
+      step[u] = softplus_f32(__bfloat162float(dt_next[u]) + bias);
+      g[u] = __bfloat162float(z_next[u]);
+    }
+    ask(t0 + SEG_AHEAD);
+#pragma unroll
+    for (int u = 0; u < SEG_AHEAD; ++u) {
+      const int t = t0 + u;
+      if (t >= tokens) break;
+      const float dx = step[u] * xv[u];
+      const float2 dx2 = make_float2(dx, dx), dt2 = make_float2(step[u], step[u]);
+      float2 acc[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+#pragma unroll
+      for (int q = 0; q < SEG_STATE / 4; ++q) {
+        const float4 bv = *reinterpret_cast<const float4 *>(&s_b[t][4 * q]);
+        float4 cv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if constexpr (!SUMS) cv = *reinterpret_cast<const float4 *>(&s_c[t][4 * q]);
+        S[2 * q] = __ffma2_rn(exp_pair(__fmul2_rn(dt2, a[2 * q])), S[2 * q], __fmul2_rn(dx2, make_float2(bv.x, bv.y)));
+        S[2 * q + 1] = __ffma2_rn(exp_pair(__fmul2_rn(dt2, a[2 * q + 1])), S[2 * q + 1], __fmul2_rn(dx2, make_float2(bv.z, bv.w)));
+        if constexpr (!SUMS) {
+          acc[0] = __ffma2_rn(S[2 * q], make_float2(cv.x, cv.y), acc[0]);
+          acc[1] = __ffma2_rn(S[2 * q + 1], make_float2(cv.z, cv.w), acc[1]);
+        }
+      }
+      if constexpr (SUMS) {
+        sum += step[u];
+      } else {
+        float y = fmaf(d_skip, xv[u], (acc[0].x + acc[0].y) + (acc[1].x + acc[1].y));
+        if (zs != nullptr) y *= g[u] / (1.0f + expf(-g[u]));
+        outs[t * p.out_stride] = le::from_f32<TO>(y * p.out_scale);
+      }
+    }
+  }
+  float *to = SUMS ? piece : (last ? kept : nullptr);
+  if (SUMS) s.sums[static_cast<int64_t>(seg) * p.rows + row] = sum;
+  if (to != nullptr) {
+#pragma unroll
+    for (int n = 0; n < SEG_STATE; n += 2) {
+      if (n < N) to[n] = S[n / 2].x;
+      if (n + 1 < N) to[n + 1] = S[n / 2].y;
+    }
+  }
+}
+
+// A thread per number of a row's state, a block row per segment: those at a request's first segment walk down its others.
+__global__ void __launch_bounds__(256)
+selective_starts_kernel(SsmArgs p, SegArgs s, int num_segments) {
+  le::let_successor_start();
+  const int seg = blockIdx.y;
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
+  const int64_t all = static_cast<int64_t>(p.rows) * p.n_state;
+  if (s.tile_q0[seg] != 0 || i >= all) return;
+  const int b = s.tile_request[seg];
+  const int segments = (p.cu_q[b + 1] - p.cu_q[b] + SEG_TOKENS - 1) / SEG_TOKENS;
+  const int slot = p.state_slots[b];
+  const bool has_state = slot >= 0 && slot < p.num_state_rows;
+  const int64_t row = i / p.n_state;
+  const float rate = -expf(p.a_log[i]);
+  le::wait_for_predecessor();
+  float S = has_state ? p.state[static_cast<int64_t>(slot) * all + i] : 0.0f;
+  int at = seg;                                  // the request's next segment in the list
+  constexpr int AHEAD = 8;
+  for (int s0 = 0; s0 < segments; s0 += AHEAD) {
+    float own[AHEAD], sum[AHEAD];
+    int where[AHEAD];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      while (at < num_segments && s.tile_request[at] != b) ++at;
+      where[u] = s0 + u < segments && at < num_segments ? at++ : -1;
+      own[u] = sum[u] = 0.0f;
+      if (where[u] >= 0 && s0 + u + 1 < segments) {       // (the last segment has no sums, and nothing follows it)
+        own[u] = s.scratch[where[u] * all + i];
+        sum[u] = s.sums[static_cast<int64_t>(where[u]) * p.rows + row];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      if (where[u] < 0) break;
+      s.scratch[where[u] * all + i] = S;
+      S = fmaf(le::exp_unbiased(rate * sum[u]), S, own[u]);
+    }
+  }
+}
+
 template <typename T, typename TO, int NPER, int LANES>
 int launch_ssm(const SsmArgs &p, int per_row, int num_requests, cudaStream_t stream) {
   const int rows_per_block = p.rows_per_block;
@@ -342,4 +580,39 @@ LE_API int le_ssm_scan(void *out, int out_dtype, int64_t out_stride, const void 
   if (dtype == LE_BF16 && out_dtype == LE_BF16) LE_SSM(__nv_bfloat16, __nv_bfloat16);
 #undef LE_SSM
   return le::invalid("le_ssm_scan: no form for input type %d and output type %d", dtype, out_dtype);
+}
+
+LE_API int le_selective_segment() { return SEG_TOKENS; }
+LE_API int le_selective_max_state() { return SEG_STATE; }
+
+// le_ssm_scan's form with a decay per row and state over segments of le_selective_segment() tokens, for bfloat16 rows
+// of one group and up to le_selective_max_state() numbers of state per row.  tile_request / tile_q0 list num_segments
+// segments: their requests and their first tokens within them, a request's segments in their order.  scratch: float32
+// [num_segments, rows, n_state + 1] where a request has several segments, else null.
+LE_API int le_selective_segments(void *out, int out_dtype, int64_t out_stride, const void *x, int64_t x_stride, const void *bc,
+                                 int64_t bc_stride, int b_col, int c_col, const void *dt, int64_t dt_stride, const void *z,
+                                 int64_t z_stride, const float *dt_bias, const float *a_log, const float *d_skip, float *state,
+                                 int num_state_rows, const int32_t *state_slots, const int32_t *cu_q,
+                                 const int32_t *tile_request, const int32_t *tile_q0, int num_segments, int rows, int n_state,
+                                 float out_scale, float *scratch, cudaStream_t stream) {
+  if (num_segments <= 0 || rows <= 0) return 0;
+  if (num_segments > 65535) return le::invalid("le_selective_segments: too many segments for one launch");
+  if (n_state < 1 || n_state > SEG_STATE) return le::invalid("le_selective_segments: %d numbers of state per row (1..%d)", n_state, SEG_STATE);
+  if (out_dtype != LE_BF16 && out_dtype != LE_F32) return le::invalid("le_selective_segments: unknown dtype code %d", out_dtype);
+  SsmArgs p{};
+  p.x = x, p.x_stride = x_stride, p.bc = bc, p.bc_stride = bc_stride, p.b_col = b_col, p.c_col = c_col;
+  p.dt = dt, p.dt_stride = dt_stride, p.z = z, p.z_stride = z_stride, p.out = out, p.out_stride = out_stride;
+  p.dt_bias = dt_bias, p.a_log = a_log, p.d_skip = d_skip, p.state = state, p.num_state_rows = num_state_rows;
+  p.state_slots = state_slots, p.cu_q = cu_q, p.rows = rows, p.n_state = n_state, p.out_scale = out_scale;
+  SegArgs s{tile_request, tile_q0, scratch, scratch != nullptr ? scratch + static_cast<int64_t>(num_segments) * rows * n_state : nullptr};
+  const dim3 grid((rows + SEG_THREADS - 1) / SEG_THREADS, num_segments);
+  if (scratch != nullptr) {
+    int rc = le::launch_chained(selective_segment_kernel<float, true>, grid, dim3(SEG_THREADS), 0, stream, p, s);
+    if (rc != 0) return rc;
+    const dim3 starts(static_cast<unsigned>((static_cast<int64_t>(rows) * n_state + 255) / 256), num_segments);
+    rc = le::launch_chained(selective_starts_kernel, starts, dim3(256), 0, stream, p, s, num_segments);
+    if (rc != 0) return rc;
+  }
+  if (out_dtype == LE_F32) return le::launch_chained(selective_segment_kernel<float, false>, grid, dim3(SEG_THREADS), 0, stream, p, s);
+  return le::launch_chained(selective_segment_kernel<__nv_bfloat16, false>, grid, dim3(SEG_THREADS), 0, stream, p, s);
 }

@@ -113,6 +113,11 @@ _CORE_SIGNATURES = {
     "le_ssm_scan": [c_void_p, c_int, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_void_p, c_int64, c_void_p,
                     c_int64, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
                     c_int, c_int, c_int, c_int, c_int, c_float, c_void_p],
+    "le_selective_segment": [],
+    "le_selective_max_state": [],
+    "le_selective_segments": [c_void_p, c_int, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_void_p, c_int64,
+                              c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
+                              c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
     "le_decay_segment": [],
     "le_duality_chunks": [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_void_p, c_int64, c_void_p,
                           c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
@@ -1674,8 +1679,46 @@ def ssm_scan(out, x, bc, b_col: int, c_col: int, dt, z, dt_bias, a_log, d_skip, 
                               int(rows_per_group), 1 if per_row else 0, float(out_scale), _stream()), "le_ssm_scan")
 
 
-DECAY_CHUNK_MAX_DIM = 128          # entries of a head's keys that the forms over chunks take
 _segment_sizes: dict[str, int] = {}
+SELECTIVE_MAX_STATE = 16           # numbers of state per row that the form over segments takes
+
+
+def selective_segment() -> int:
+    """Tokens per segment of selective_segments()."""
+    if "selective" not in _segment_sizes:
+        _segment_sizes["selective"] = int(core().le_selective_segment())
+    return _segment_sizes["selective"]
+
+
+def selective_segments(out, x, bc, b_col: int, c_col: int, dt, z, dt_bias, a_log, d_skip, state, state_slots, cu_q, tile_request,
+                       tile_q0, num_segments: int, n_state: int, scratch, out_scale: float = 1.0) -> None:
+    """ssm_scan() with a decay per row and state over segments side by side,
+    for the requests whose segments (selective_segment() tokens each, a
+    request's in their order) the first ``num_segments`` entries of the tile
+    lists name.  Rows bfloat16 and of one group, ``out`` that type or float32,
+    at most SELECTIVE_MAX_STATE numbers of state per row.  ``scratch``:
+    float32 [num_segments, rows, n_state + 1] where a request has several
+    segments, else None."""
+    _need_cuda(out, x, bc, dt, z, dt_bias, a_log, d_skip, state, state_slots, cu_q, tile_request, tile_q0, scratch)
+    T, rows = x.shape
+    assert out.shape == (T, rows) and out.stride(1) == 1 and x.stride(1) == 1 and bc.stride(1) == 1 and dt.stride(1) == 1
+    assert x.dtype == bc.dtype == dt.dtype == torch.bfloat16 and dt.shape == (T, rows)
+    assert z is None or (z.dtype == x.dtype and z.stride(1) == 1 and z.shape == x.shape)
+    assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (rows, n_state)
+    assert n_state <= SELECTIVE_MAX_STATE and dt_bias.dtype == a_log.dtype == torch.float32 and a_log.is_contiguous()
+    assert dt_bias.numel() == rows and a_log.numel() == rows * n_state
+    assert d_skip is None or (d_skip.dtype == torch.float32 and d_skip.numel() == rows)
+    assert scratch is None or (scratch.dtype == torch.float32 and scratch.is_contiguous()
+                               and scratch.numel() >= num_segments * rows * (n_state + 1))
+    _check(core().le_selective_segments(_ptr(out), dtype_code(out.dtype), out.stride(0), _ptr(x), x.stride(0), _ptr(bc),
+                                        bc.stride(0), int(b_col), int(c_col), _ptr(dt), dt.stride(0), _ptr(z),
+                                        z.stride(0) if z is not None else 0, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
+                                        _ptr(state), state.shape[0], _ptr(state_slots), _ptr(cu_q), _ptr(tile_request),
+                                        _ptr(tile_q0), int(num_segments), rows, int(n_state), float(out_scale), _ptr(scratch),
+                                        _stream()), "le_selective_segments", launches=1 if scratch is None else 3)
+
+
+DECAY_CHUNK_MAX_DIM = 128          # entries of a head's keys that the forms over chunks take
 
 
 def decay_segment() -> int:

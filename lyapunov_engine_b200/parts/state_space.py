@@ -21,8 +21,9 @@ G)), inner = H * P:
 
 Both recurrences run in one kernel (ops.ssm_scan), with the gate in its
 epilogue; requests that bring several tokens in bfloat16 go through the duality
-over chunks on the tensor cores instead (ops.duality_chunks).  The convolution is the package's short convolution with a bias and
-silu; the last taps - 1 inputs of the convolution are state of the request too
+over chunks on the tensor cores (ops.duality_chunks) and through the selective
+scan over segments side by side (ops.selective_segments) instead.  The
+convolution is the package's short convolution with a bias and silu; the last taps - 1 inputs of the convolution are state of the request too
 (``extra_state_needs``).  Step sizes, decays, the recurrence and the norm are
 32-bit.
 """
@@ -33,6 +34,7 @@ import torch
 from .. import ops
 from .base import Mixer, StateNeed, TensorDecl, register_mixer
 
+SELECTIVE_SEGMENT = 64   # tokens of a request that a block of the selective scan's form over segments takes
 SEGMENT = 256      # tokens of a request that a block of the duality's chunked form takes
 
 
@@ -187,7 +189,7 @@ class SelectiveScanMixer(Mixer):
         return {"mixer_taps": StateNeed((self.taps - 1, self.channels), torch.float32)}
 
     def tile_sizes(self):
-        return [ops.SHORT_CONV_TILE]
+        return [ops.SHORT_CONV_TILE, SELECTIVE_SEGMENT]
 
     def tensors(self):
         W, C, N, R = self.hidden_size, self.inner, self.state_dim, self.dt_rank
@@ -215,6 +217,8 @@ class SelectiveScanMixer(Mixer):
         self.w_dt[:, :R] = wdt
         self.dt_bias, self.a_log, self.d_skip = get(self.dt_bias_name), get(self.a_log_name).contiguous(), get(self.d_name)
         self.w_o = get(self.o_name)
+        if ops.selective_segment() != SELECTIVE_SEGMENT:
+            raise RuntimeError(f"the kernels' segments have {ops.selective_segment()} tokens, the mixer lists {SELECTIVE_SEGMENT}")
         self.runtime = runtime
 
     def inner_width(self) -> int:
@@ -241,7 +245,17 @@ class SelectiveScanMixer(Mixer):
         ops.linear(dt, low, self.w_dt, ctx.status)
         if out is None:
             out = ws.get("scan_gated", (T, C), rt.dtype)
-        ops.ssm_scan(out, conv, low, self.b_col, self.c_col, dt, proj[:, self.z_col:self.z_col + C], self.dt_bias, self.a_log,
-                     self.d_skip, cache.state, ctx.state_slots, ctx.cu_q, ctx.num_requests, N, 1, C, per_row=True,
-                     out_scale=scale)
+        rows = (out, conv, low, self.b_col, self.c_col, dt, proj[:, self.z_col:self.z_col + C], self.dt_bias, self.a_log,
+                self.d_skip, cache.state, ctx.state_slots, ctx.cu_q)
+        request, q0, _, segments = ctx.tiles[SELECTIVE_SEGMENT]
+        if segments and rt.dtype == torch.bfloat16 and N <= ops.SELECTIVE_MAX_STATE:
+            # (a step in which no request has a second segment goes from state row to state row)
+            scratch = None
+            if segments > ctx.num_requests - ctx.num_decode:
+                scratch = ws.get("scan_scratch", (segments, C, N + 1), torch.float32)
+            ops.selective_segments(*rows, request, q0, segments, N, scratch, out_scale=scale)
+            if ctx.num_decode:
+                ops.ssm_scan(*rows, ctx.num_decode, N, 1, C, per_row=True, out_scale=scale, requests=ctx.decode_requests)
+        else:
+            ops.ssm_scan(*rows, ctx.num_requests, N, 1, C, per_row=True, out_scale=scale)
         return out
