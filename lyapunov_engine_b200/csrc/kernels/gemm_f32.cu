@@ -4,7 +4,27 @@
 //
 // Every output element is one chain of fused multiply-adds over k = 0 .. K-1
 // in ascending order, so a token's projections are bit-for-bit the same
-// whichever rows share its step and wherever its row lies in the batch.
+// whichever rows share its step, wherever its row lies in the batch, and
+// whichever form below computes them.
+//
+// gemm_f32_kernel takes float32 operands whose rows are whole 16-byte pieces.
+// A block's 128 threads stand in TY rows; a thread computes RM x RN outputs in
+// registers.  Operands flow through a ring of shared-memory stages (cp.async,
+// KB of k each, as they lie in memory, no transposition): a thread reads four
+// k of a row at a time, rows of a stage are KB + 4 floats apart, and a thread's
+// rows lie TY (of A) or 128 / TY (of W) apart, so that the eight threads of a
+// quarter-warp read eight neighbouring rows of W from different banks.
+// What bounds it: many rows, the FMA pipes and next to them the shared-memory
+// reads, RM + RN of 16 bytes per 4 RM RN multiply-adds (336 rows, 16,384 x
+// 2,048: 582 us, 52 % of the pipes' 74 TFLOP/s, against 1,058 in the general
+// form, whose loads of single floats are uncoalesced and whose 4 x 4 outputs a
+// thread need twice the reads); few rows, the bytes of W (4 rows, 128,256 x
+// 2,048: 205 us, 5.1 TB/s, against 1,175), or, where W has few rows, the chain
+// of K dependent multiply-adds (8 rows, 2,048 x 8,192: 62 us, against 635).
+// Tiles turned to [k][row] with pairs of columns in packed multiply-adds were
+// no faster (584 us) and slower with few blocks (498 against 409 us).
+//
+// gemm_simt_kernel takes everything else (bfloat16 operands, odd strides).
 //
 // The reference has no matrix-product kernel: its projections are nn.Linear
 // (python/lyapunov_engine/models/llama.py:45-48,112-117,177).
@@ -12,6 +32,7 @@
 
 namespace {
 
+// ---- the general form
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
 
 template <typename TI, typename TC>
@@ -65,6 +86,160 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(TC *__restrict__ C, cons
   }
 }
 
+// ---- float32 operands in 16-byte pieces
+constexpr int F32_THREADS = 128;      // 8 rows of threads by 16 columns of threads
+
+__device__ __forceinline__ void cp16(float *smem, const float *gmem, bool valid) {
+  const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  const int bytes = valid ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(gmem), "r"(bytes));
+}
+
+template <int TY, int RM, int RN, int KB, int STAGES>
+struct F32Tile {
+  static constexpr int BM = TY * RM, BN = F32_THREADS / TY * RN, PITCH = KB + 4;
+  static constexpr int A_STAGE = BM * PITCH, STAGE = (BM + BN) * PITCH;
+  static constexpr size_t SMEM = sizeof(float) * STAGES * STAGE;
+};
+
+template <int TY, int RM, int RN, int KB, int STAGES>
+__global__ void __launch_bounds__(F32_THREADS)
+gemm_f32_kernel(float *__restrict__ C, const float *__restrict__ A, const float *__restrict__ W, int M, int N, int K,
+                int64_t lda, int64_t ldw, int64_t ldc) {
+  using Tile = F32Tile<TY, RM, RN, KB, STAGES>;
+  extern __shared__ __align__(16) float f32_smem[];
+  constexpr int PITCH = Tile::PITCH, CPR = KB / 4;       // 16-byte pieces per row of a stage
+  const int tid = threadIdx.x;
+  // a warp is 4 rows of threads by 8 columns of threads
+  const int warp = tid >> 5, lane = tid & 31;
+  constexpr int TX = F32_THREADS / TY;
+  const int ty = TY == 8 ? (warp >> 1) * 4 + (lane >> 3) : tid / TX, tx = TY == 8 ? (warp & 1) * 8 + (lane & 7) : tid % TX;
+  const int m0 = blockIdx.y * Tile::BM, n0 = blockIdx.x * Tile::BN;
+  const int num_tiles = (K + KB - 1) / KB;
+
+  auto load = [&](int s, int kt) {
+    float *dst = f32_smem + s * Tile::STAGE;
+    constexpr int A_PIECES = Tile::BM * CPR, PIECES = (Tile::BM + Tile::BN) * CPR;
+#pragma unroll
+    for (int i = 0; i < (PIECES + F32_THREADS - 1) / F32_THREADS; ++i) {
+      const int c = tid + i * F32_THREADS;
+      if (PIECES % F32_THREADS != 0 && c >= PIECES) break;
+      const int row = c / CPR, k = kt * KB + (c % CPR) * 4;
+      const bool is_a = c < A_PIECES;
+      const int64_t r = is_a ? m0 + row : n0 + row - Tile::BM;
+      const bool valid = r < (is_a ? M : N) && k < K;
+      const float *src = is_a ? A + (valid ? r * lda + k : 0) : W + (valid ? r * ldw + k : 0);
+      cp16(dst + row * PITCH + (c % CPR) * 4, src, valid);
+    }
+  };
+
+  float acc[RM][RN];
+#pragma unroll
+  for (int i = 0; i < RM; ++i)
+#pragma unroll
+    for (int j = 0; j < RN; ++j) acc[i][j] = 0.0f;
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) {
+    if (s < num_tiles) load(s, s);
+    asm volatile("cp.async.commit_group;\n" ::);
+  }
+  for (int kt = 0; kt < num_tiles; ++kt) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2));
+    __syncthreads();
+    const int next = kt + STAGES - 1;
+    if (next < num_tiles) load(next % STAGES, next);
+    asm volatile("cp.async.commit_group;\n" ::);
+    const float *as = f32_smem + (kt % STAGES) * Tile::STAGE + ty * PITCH;
+    const float *ws = f32_smem + (kt % STAGES) * Tile::STAGE + Tile::A_STAGE + tx * PITCH;
+#pragma unroll(RM *RN >= 32 ? 2 : 4)
+    for (int k = 0; k < KB; k += 4) {
+      float4 a[RM], w[RN];
+#pragma unroll
+      for (int i = 0; i < RM; ++i) a[i] = *reinterpret_cast<const float4 *>(as + i * TY * PITCH + k);
+#pragma unroll
+      for (int j = 0; j < RN; ++j) w[j] = *reinterpret_cast<const float4 *>(ws + j * TX * PITCH + k);
+#pragma unroll
+      for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < RN; ++j) acc[i][j] = fmaf(a[i].x, w[j].x, acc[i][j]);
+#pragma unroll
+      for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < RN; ++j) acc[i][j] = fmaf(a[i].y, w[j].y, acc[i][j]);
+#pragma unroll
+      for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < RN; ++j) acc[i][j] = fmaf(a[i].z, w[j].z, acc[i][j]);
+#pragma unroll
+      for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < RN; ++j) acc[i][j] = fmaf(a[i].w, w[j].w, acc[i][j]);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::);
+#pragma unroll
+  for (int i = 0; i < RM; ++i) {
+    const int m = m0 + ty + TY * i;
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < RN; ++j) {
+      const int n = n0 + tx + TX * j;
+      if (n < N) C[m * ldc + n] = acc[i][j];
+    }
+  }
+}
+
+template <int TY, int RM, int RN, int KB, int STAGES>
+int launch_f32(float *C, const float *A, const float *W, int M, int N, int K, int64_t lda, int64_t ldw, int64_t ldc,
+               cudaStream_t stream) {
+  using Tile = F32Tile<TY, RM, RN, KB, STAGES>;
+  auto kernel = gemm_f32_kernel<TY, RM, RN, KB, STAGES>;
+  if (Tile::SMEM > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Tile::SMEM));
+    if (e != cudaSuccess) return le::invalid("le_gemm_simt: cannot get %zu bytes of shared memory: %s", Tile::SMEM, cudaGetErrorString(e));
+  }
+  const dim3 grid((N + Tile::BN - 1) / Tile::BN, (M + Tile::BM - 1) / Tile::BM);
+  kernel<<<grid, F32_THREADS, Tile::SMEM, stream>>>(C, A, W, M, N, K, lda, ldw, ldc);
+  return le::launched();
+}
+
+// The tile shapes, and what a product costs with each: `base` + `per_round` for every round of blocks (one a
+// multiprocessor; blocks beyond the first share its pipes), in microseconds at K = 2,048, of which both are multiples.
+// Fitted to 1 .. 520 rows against 2,048, 3,072, 16,384 and 128,256 columns; the least is within a tenth of the best of
+// 20 shapes measured at all but two of 41 sizes (within a quarter there).
+struct F32Shape {
+  int bm, bn;
+  float base, per_round;
+  decltype(&launch_f32<8, 1, 1, 64, 8>) launch;
+};
+constexpr F32Shape F32_SHAPES[] = {
+    {4, 64, 18.0f, 13.0f, launch_f32<2, 2, 1, 64, 4>},    {8, 16, 15.0f, 7.0f, launch_f32<8, 1, 1, 64, 8>},
+    {8, 32, 15.0f, 9.5f, launch_f32<4, 2, 1, 64, 5>},     {8, 64, 25.0f, 15.0f, launch_f32<2, 4, 1, 32, 4>},
+    {16, 16, 12.0f, 10.0f, launch_f32<8, 2, 1, 64, 6>},   {16, 64, 25.0f, 19.5f, launch_f32<4, 4, 2, 32, 4>},
+    {32, 32, 18.0f, 21.0f, launch_f32<8, 4, 2, 32, 4>},   {32, 64, 28.0f, 29.5f, launch_f32<8, 4, 4, 32, 4>},
+    {48, 64, 33.0f, 42.0f, launch_f32<8, 6, 4, 16, 4>},   {64, 128, 48.0f, 100.0f, launch_f32<8, 8, 8, 32, 3>},
+};
+
+int multiprocessors() {
+  int device = 0, sms = 0;
+  if (cudaGetDevice(&device) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0) return sms;
+  cudaGetLastError();
+  return 148;
+}
+
+const F32Shape *best_shape(int M, int N) {
+  static const int sms = multiprocessors();
+  const F32Shape *best = nullptr;
+  float least = 0.0f;
+  for (const F32Shape &s : F32_SHAPES) {
+    const int64_t rows = (static_cast<int64_t>(M) + s.bm - 1) / s.bm, blocks = rows * ((static_cast<int64_t>(N) + s.bn - 1) / s.bn);
+    if (rows > 65535) continue;
+    const float cost = s.base + s.per_round * static_cast<float>((blocks + sms - 1) / sms);
+    if (best == nullptr || cost < least) best = &s, least = cost;
+  }
+  return best;
+}
+
 }  // namespace
 
 // Inputs of one type (f32 or bf16), 32-bit accumulation, output f32 or bf16.
@@ -73,6 +248,11 @@ LE_API int le_gemm_simt(void *C, int c_dtype, const void *A, const void *W, int 
                         int64_t lda, int64_t ldw, int64_t ldc, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return le::invalid("le_gemm_simt: K must be positive");
+  const bool pieces = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
+  if (in_dtype == LE_F32 && c_dtype == LE_F32 && pieces) {
+    if (const F32Shape *shape = best_shape(M, N))
+      return shape->launch(static_cast<float *>(C), static_cast<const float *>(A), static_cast<const float *>(W), M, N, K, lda, ldw, ldc, stream);
+  }
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   if (grid.y > 65535) return le::invalid("le_gemm_simt: M = %d is too large for one launch", M);
 #define LE_GO(TI, TC) gemm_simt_kernel<TI, TC><<<grid, 256, 0, stream>>>(static_cast<TC *>(C), static_cast<const TI *>(A), static_cast<const TI *>(W), M, N, K, lda, ldw, ldc)
