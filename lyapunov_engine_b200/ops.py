@@ -1365,8 +1365,10 @@ GATED_DELTA_MAX_DIM = 1024
 
 
 def gated_delta_scratch_width(heads: int, kv_heads: int) -> int:
-    """Floats per token of the scratch rows that ``gated_delta_scan`` fills (inverse lengths, k . q, decay, step size)."""
-    return 4 * int(kv_heads) + 2 * int(heads)
+    """Floats per token of the scratch that ``gated_delta_scan`` fills
+    (inverse lengths, products of neighbouring tokens' unit vectors, decay,
+    step size, and what groups of tokens make of them)."""
+    return int(core().le_gated_delta_scratch(int(heads), int(kv_heads)))
 
 
 def gated_delta_scan(out, qkv, q_col, k_col, v_col, proj, b_col, a_col, a_log, dt_bias, state, state_slots, cu_q,
