@@ -21,10 +21,8 @@ namespace {
 
 constexpr int THREADS = 1024;
 
-__device__ __forceinline__ uint32_t ordered_key(float x) {
-  const uint32_t u = __float_as_uint(x);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
+__device__ __forceinline__ uint32_t ordered_key(uint32_t u) { return (u & 0x80000000u) ? ~u : (u | 0x80000000u); }
+__device__ __forceinline__ uint32_t ordered_key(float x) { return ordered_key(__float_as_uint(x)); }
 
 __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
   x += 0x9E3779B97F4A7C15ull;
@@ -126,7 +124,10 @@ __global__ void argmax_final_kernel(int32_t *__restrict__ out, const float *__re
 // memory once, and every later pass runs from there.  The blocks exchange what they find through distributed
 // shared memory.
 //
-// The two thresholds need no sort: radix selection over the ordered bit patterns, 11 + 11 + 10 bits.  A level
+// The two thresholds need no sort.  First by value: bins of equal width below the row's maximum (linear_select), which
+// a row's values fall into evenly, so that plain atomic additions do; the few values of the bin that a threshold lies in
+// are then compared with one another.  Where that cannot be done (a bin with too many values, rows with NaN or infinite
+// maxima, more values to keep than there are threads) by radix selection over the ordered bit patterns, 11 + 11 + 10 bits.  A level
 // makes a histogram (count, and for top-p the probability mass, per digit) of the row's values whose higher
 // digits are the ones chosen so far; block 0 adds the blocks' histograms up and picks the digit the threshold
 // lies in.  Masses are fixed-point integers (2^-40 of the largest probability), so that sums do not depend on
@@ -154,8 +155,16 @@ struct SampleShared {
   int count_above;
   unsigned long long mass_above;
   unsigned long long mass_limit;
+  // linear_select: one entry for each of a row's two thresholds where a block may be a selection ahead of another
+  unsigned long long share[2];             // the sum over this block's share of the bins
+  unsigned long long above;                // what lies above the bin the threshold falls into, and that bin
+  int bin;
+  int listed[2];                           // block 0: values of that bin
+  uint32_t chosen[2];                      // block 0: the threshold
   // what every block tells the others
   float block_max;
+  float block_floor;                       // the smallest of the threads' maxima
+  int block_odd;                           // a NaN was seen
   int block_argmax;
   float block_total;
   float block_z;
@@ -319,6 +328,113 @@ __device__ uint32_t radix_select(cg::cluster_group &cluster, SampleShared &h, Me
   return prefix > min_key ? prefix : min_key;
 }
 
+// The same thresholds by value.  Bin b holds the values x with floor((row_max - x) * scale) = b (the last one also all
+// below): every block's histogram, sums over all blocks' (a block takes an eighth of the bins), the bin the threshold
+// falls into, its values into a list in block 0, and there the threshold: of the values whose sum above stays within the
+// limit the smallest.  `limit`: top_p of all mass, or k - 1.  The first levels of the radix selection put a row's values
+// into some 40 bins (sign, exponent, two bits): a warp's lanes had to be sorted out by bin before they could add, twelve
+// groups one after the other, which was the time of a row with top_p (one row of 128,256: 92 us, of which a row without
+// filters takes 17; now 27).  False: the radix selection has to do it.
+constexpr int LIST_MAX = 512;              // (every value of the list meets every other)
+struct BinList {
+  unsigned long long mass[LIST_MAX];
+  uint32_t key[LIST_MAX];
+};
+static_assert(sizeof(BinList) <= sizeof(MergedHistogram), "the list lies where the merged histogram does");
+
+__device__ bool linear_select(cg::cluster_group &cluster, SampleShared &h, BinList *list, int which, const float *vals, int n,
+                              bool with_mass, int k, float top_p, uint32_t min_key, float row_max, float inv_t, float scale,
+                              uint32_t &threshold) {
+  constexpr int SHARE = RADIX_BINS / SAMPLE_BLOCKS;
+  const int rank = static_cast<int>(cluster.block_rank()), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto bin_of = [&](float x) { return static_cast<int>(fminf((row_max - x) * scale, static_cast<float>(RADIX_BINS - 1))); };
+  auto mass_of = [&](float x) -> unsigned long long { return with_mass ? __float2ull_rd(prob_of(x, row_max, inv_t) * MASS_ONE) : 1ull; };
+  for (int bin = threadIdx.x; bin < RADIX_BINS; bin += blockDim.x) h.mass_lo[bin] = 0, h.mass_hi[bin] = 0;
+  if (threadIdx.x == 0) h.listed[which] = 0, h.chosen[which] = 0xffffffffu;
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const float x = vals[i];
+    if (ordered_key(x) < min_key) continue;
+    const unsigned long long m = mass_of(x);
+    if (m == 0) continue;
+    const int bin = bin_of(x);
+    const unsigned add_lo = static_cast<unsigned>(m), add_hi = static_cast<unsigned>(m >> 32);
+    const unsigned old = atomicAdd(&h.mass_lo[bin], add_lo);
+    const unsigned carry = old + add_lo < old ? 1u : 0u;              // additions with carry commute: the sum is exact
+    if (add_hi + carry) atomicAdd(&h.mass_hi[bin], add_hi + carry);
+  }
+  cluster.sync();                          // every block's histogram is there
+  // this block's share of the bins, summed over the blocks and scanned: warps 0 .. SHARE / 32 - 1, a bin a lane
+  unsigned long long mine = 0, upto = 0;
+  const int my_bin = rank * SHARE + static_cast<int>(threadIdx.x);
+  if (threadIdx.x < SHARE) {
+#pragma unroll
+    for (int other = 0; other < SAMPLE_BLOCKS; ++other) {
+      const SampleShared *theirs = cluster.map_shared_rank(&h, other);
+      mine += (static_cast<unsigned long long>(theirs->mass_hi[my_bin]) << 32) + theirs->mass_lo[my_bin];
+    }
+    upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long below = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += below;
+    }
+    if (lane == 31) h.warp_mass[warp] = upto;
+  }
+  __syncthreads();
+  if (threadIdx.x < SHARE) {
+    for (int w = 0; w < warp; ++w) upto += h.warp_mass[w];
+    if (threadIdx.x == SHARE - 1) h.share[which] = upto;
+  }
+  cluster.sync();                          // every block's share is summed
+  unsigned long long total = 0, before = 0;
+  for (int other = 0; other < SAMPLE_BLOCKS; ++other) {
+    if (other == rank) before = total;
+    total += cluster.map_shared_rank(&h, other)->share[which];
+  }
+  const unsigned long long limit = with_mass ? __double2ull_rd(static_cast<double>(top_p) * static_cast<double>(total))
+                                             : static_cast<unsigned long long>(k - 1);
+  if (total <= limit) return false;        // (every block sees the same)
+  if (threadIdx.x < SHARE && before + upto - mine <= limit && before + upto > limit) h.bin = my_bin, h.above = before + upto - mine;
+  int owner = -1;                          // the last block up to whose share the sum stays within the limit
+  for (unsigned long long sum = 0; owner + 1 < SAMPLE_BLOCKS && sum <= limit;) sum += cluster.map_shared_rank(&h, ++owner)->share[which];
+  cluster.sync();                          // the owner of that bin has found it
+  const SampleShared *from = cluster.map_shared_rank(&h, owner);
+  const int bin = from->bin;
+  const unsigned long long above = from->above;
+  SampleShared *first = cluster.map_shared_rank(&h, 0);
+  BinList *all = cluster.map_shared_rank(list, 0);
+  const int rounds = (n + blockDim.x - 1) / blockDim.x;
+  for (int round = 0; round < rounds; ++round) {
+    const int i = round * blockDim.x + threadIdx.x;
+    const float x = i < n ? vals[i] : 0.0f;
+    bool in = i < n && ordered_key(x) >= min_key && bin_of(x) == bin;
+    unsigned long long m = 0;
+    if (in) m = mass_of(x), in = m != 0;   // (a value without mass is no threshold)
+    const unsigned found = __ballot_sync(0xffffffffu, in);
+    if (found == 0) continue;
+    int at = 0;
+    if (lane == 0) at = atomicAdd(&first->listed[which], __popc(found));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(found & ((1u << lane) - 1u));
+    if (in && at < LIST_MAX) all->key[at] = ordered_key(x), all->mass[at] = m;
+  }
+  cluster.sync();                          // the list is complete
+  const int listed = first->listed[which];
+  if (listed > LIST_MAX) {
+    cluster.sync();                        // (nobody clears the list's place while another still reads its length)
+    return false;
+  }
+  if (rank == 0 && threadIdx.x < listed) {
+    const uint32_t key = list->key[threadIdx.x];
+    unsigned long long sum = above;
+    for (int i = 0; i < listed; ++i) sum += list->key[i] > key ? list->mass[i] : 0ull;
+    if (sum <= limit) atomicMin(&h.chosen[which], key);
+  }
+  cluster.sync();
+  threshold = max(first->chosen[which], min_key);
+  return true;
+}
+
 // An inclusive prefix sum over the block's threads in thread order (fixed tree: the same bits every time).
 __device__ float block_inclusive_scan(float v, float *warp_f, float &block_total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (blockDim.x + 31) >> 5;
@@ -345,8 +461,13 @@ __device__ float block_inclusive_scan(float v, float *warp_f, float &block_total
 }
 
 // params per row: temperature, top_p (floats), top_k, seed_lo, seed_hi, counter (ints).
+// TO_A_SM: blocks a multiprocessor is to hold.  Two (32 registers a thread, some 40 spilled) where there are more blocks
+// than multiprocessors: the waits of one block's meetings are the other's time (64 rows of 128,256 with all kinds of options:
+// 234 us before the selection by value, 107 with it, 96 with two blocks).  One otherwise (a row with top_p 27 us, with
+// 32 registers 31).
 // slice: values per block (a multiple of 4); `staged`: the slice fits in shared memory and is copied there.
-__global__ void __launch_bounds__(THREADS)
+template <int TO_A_SM>
+__global__ void __launch_bounds__(THREADS, TO_A_SM)
 sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int vocab, int64_t stride, int slice, int staged,
               const float *__restrict__ temperature, const float *__restrict__ top_p, const int32_t *__restrict__ top_k,
               const int32_t *__restrict__ seeds, const float *__restrict__ uniforms, float *__restrict__ probs_out) {
@@ -362,6 +483,9 @@ sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int v
   const int begin = min(vocab, rank * slice);
   const int n = min(slice, vocab - begin);
   const float temp = temperature[r];
+  const int k = top_k[r];
+  const float p_keep = top_p[r];
+  const bool filtered = !(temp < 1e-4f) && ((k > 0 && k < vocab) || p_keep < 1.0f);
 
   // ---- this block's slice into shared memory; its maximum (first index on ties)
   const float *vals = row + begin;
@@ -378,15 +502,23 @@ sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int v
     }
     vals = slice_smem;
   }
-  if (rank == 0)
-    for (int bin = threadIdx.x; bin < RADIX_BINS; bin += blockDim.x) { merged->count[bin] = 0; merged->mass[bin] = 0; }
   __syncthreads();
   {
     float best = -INFINITY;
     int idx = 0x7fffffff;
+    bool odd = false;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
       const float x = vals[i];
+      if (x != x) odd = true;
       if (x > best || (x == best && begin + i < idx)) { best = x; idx = begin + i; }
+    }
+    // for a row with filters: the smallest of the threads' maxima (a thread without a value stands aside; NaN: -inf)
+    if (filtered) {
+      float least = odd ? -INFINITY : (threadIdx.x < n ? best : INFINITY);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
+      odd = __any_sync(0xffffffffu, odd);
+      if (lane == 0) sh.warp_mass[warp] = (static_cast<unsigned long long>(odd) << 32) + __float_as_uint(least);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -407,15 +539,29 @@ sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int v
         if (ob > best || (ob == best && oi < idx)) { best = ob; idx = oi; }
       }
       if (lane == 0) { sh.block_max = best; sh.block_argmax = idx; }
+      if (filtered) {
+        const unsigned long long theirs = sh.warp_mass[lane < warps ? lane : 0];
+        float least = __uint_as_float(static_cast<uint32_t>(theirs));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
+        odd = __any_sync(0xffffffffu, (theirs >> 32) != 0);
+        if (lane == 0) { sh.block_floor = least; sh.block_odd = odd ? 1 : 0; }
+      }
     }
   }
   cluster.sync();
   float row_max = -INFINITY;
   int best = 0x7fffffff;
+  float row_floor = INFINITY;
+  bool odd = false;
   for (int other = 0; other < SAMPLE_BLOCKS; ++other) {
     const SampleShared *theirs = cluster.map_shared_rank(&sh, other);
     const float m = theirs->block_max;
     const int i = theirs->block_argmax;
+    if (filtered) {
+      row_floor = fminf(row_floor, theirs->block_floor);
+      odd = odd || theirs->block_odd != 0;
+    }
     if (m > row_max || (m == row_max && i < best)) { row_max = m; best = i; }
   }
   if (temp < 1e-4f) {
@@ -429,17 +575,49 @@ sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int v
 
   // ---- the thresholds: values whose ordered key is >= keep_key stay
   uint32_t keep_key = 0;
-  const int k = top_k[r];
-  if (k > 0 && k < vocab) keep_key = radix_select(cluster, sh, merged, vals, n, false, k, 1.0f, 0u, row_max, inv_t);
-  const float p_keep = top_p[r];
-  if (p_keep < 1.0f) keep_key = radix_select(cluster, sh, merged, vals, n, true, 0, p_keep, keep_key, row_max, inv_t);
+  BinList *list = reinterpret_cast<BinList *>(merged);
+  auto radix = [&](bool with_mass, int k, float p, uint32_t min_key) {
+    if (rank == 0)
+      for (int bin = threadIdx.x; bin < RADIX_BINS; bin += blockDim.x) { merged->count[bin] = 0; merged->mass[bin] = 0; }
+    cluster.sync();                        // (the others add to it remotely)
+    return radix_select(cluster, sh, merged, vals, n, with_mass, k, p, min_key, row_max, inv_t);
+  };
+  const bool plain = !odd && row_max < INFINITY && row_max > -INFINITY;
+  if (k > 0 && k < vocab) {
+    // From the maximum down to the smallest of the threads' maxima there are at least as many values as threads that
+    // have one.
+    const float scale = static_cast<float>(RADIX_BINS - 1) / (row_max - row_floor);
+    const int threads = min(vocab, (vocab / slice) * static_cast<int>(blockDim.x));
+    if (!(plain && k <= threads && scale > 0.0f && scale < INFINITY &&
+          linear_select(cluster, sh, list, 0, vals, n, false, k, 1.0f, 0u, row_max, inv_t, scale, keep_key)))
+      keep_key = radix(false, k, 1.0f, 0u);
+  }
+  if (p_keep < 1.0f) {
+    // a value's mass is 0 from 40 ln 2 temperatures below the maximum on
+    const float scale = static_cast<float>(RADIX_BINS - 1) / 27.8f * inv_t;
+    const uint32_t min_key = keep_key;
+    if (!(plain && scale < INFINITY &&
+          linear_select(cluster, sh, list, 1, vals, n, true, 0, p_keep, min_key, row_max, inv_t, scale, keep_key)))
+      keep_key = radix(true, 0, p_keep, min_key);
+  }
 
   // ---- the kept mass in token order: a thread takes a run of consecutive values of the slice
   const int chunk = (slice + blockDim.x - 1) / blockDim.x;
   const int c_begin = min(n, static_cast<int>(threadIdx.x) * chunk), c_end = min(n, c_begin + chunk);
   float mine = 0.0f;
   int last_kept = -1;
-  for (int i = c_begin; i < c_end; ++i)
+  // (runs of whole 16-byte pieces are read as such: single values, a run apart from lane to lane, crowd into few banks)
+  int i0 = c_begin;
+  if (staged && chunk % 4 == 0) {
+    for (; i0 + 4 <= c_end; i0 += 4) {
+      const uint4 four = *reinterpret_cast<const uint4 *>(vals + i0);
+      const uint32_t x[4] = {four.x, four.y, four.z, four.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (ordered_key(x[e]) >= keep_key) { mine += prob_of(__uint_as_float(x[e]), row_max, inv_t); last_kept = begin + i0 + e; }
+    }
+  }
+  for (int i = i0; i < c_end; ++i)
     if (ordered_key(vals[i]) >= keep_key) { mine += prob_of(vals[i], row_max, inv_t); last_kept = begin + i; }
   float mine_total;
   const float upto_me = block_inclusive_scan(mine, sh.warp_f, mine_total);   // mass of this block's threads 0 .. this one
@@ -535,8 +713,9 @@ LE_API int le_sample(int32_t *out, const float *logits, int num_rows, int vocab,
   const size_t slice_bytes = static_cast<size_t>(slice) * sizeof(float);
   const int staged = slice_bytes <= 152 * 1024 ? 1 : 0;
   const size_t smem = sizeof(MergedHistogram) + (staged ? slice_bytes : 0);
+  auto *kernel = num_rows * SAMPLE_BLOCKS > 148 ? sample_kernel<2> : sample_kernel<1>;
   {
-    cudaError_t e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return le::invalid("le_sample: cannot get %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
   }
   cudaLaunchConfig_t config = {};
@@ -551,7 +730,7 @@ LE_API int le_sample(int32_t *out, const float *logits, int num_rows, int vocab,
   attr[0].val.clusterDim.z = 1;
   config.attrs = attr;
   config.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&config, sample_kernel, out, logits, vocab, stride, slice, staged, temperature, top_p, top_k, seeds,
+  cudaError_t e = cudaLaunchKernelEx(&config, kernel, out, logits, vocab, stride, slice, staged, temperature, top_p, top_k, seeds,
                                      uniforms, probs_out);
   if (e != cudaSuccess) return le::invalid("le_sample: %s", cudaGetErrorString(e));
   return le::launched();

@@ -1,0 +1,61 @@
+"""The sampler's two thresholds on rows that its selection by value finds easy,
+hard, or leaves to the selection by bit patterns: ties in great numbers, masked
+values, flat rows, extreme temperatures, values to keep by the thousand,
+vocabularies around the sizes of slices and threads, more rows than fit at once."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+OPTIONS = [(0.8, 0.95, 0), (1.0, 1.0, 50), (0.7, 0.9, 40), (1.3, 0.5, 1000), (0.01, 0.99, 5), (1.0, 0.9999, 0), (5.0, 0.3, 3),
+           (1.0, 1e-6, 0), (100.0, 0.9, 0), (1.0, 0.9, 7000), (1.0, 0.9, 20000), (0.6, 1.0, 1), (1.0, 1.0, 8193)]
+
+
+def rows_of(kind, n, vocab, g):
+    x = torch.randn(n, vocab, generator=g, device=DEV) * 3
+    if kind == "rounded":
+        return x.bfloat16().float()
+    if kind == "flat":
+        return torch.full_like(x, 1.5)
+    if kind == "masked":
+        gone = torch.rand(n, vocab, generator=g, device=DEV) < 0.7
+        gone[:, vocab // 2] = False              # (a row without any value has no distribution)
+        return x.masked_fill(gone, -float("inf"))
+    if kind == "two":
+        return (x > 0).float()
+    if kind == "one":
+        x = torch.full_like(x, -float("inf"))
+        x[:, vocab - 1] = 2.0
+    return x
+
+
+@pytest.mark.parametrize("kind", ["normal", "rounded", "flat", "masked", "two", "one"])
+@pytest.mark.parametrize("vocab,n", [(5, 13), (1023, 13), (8200, 26), (32768, 13), (128256, 26), (300000, 13)])
+def test_kept_sets(vocab, n, kind):
+    from lyapunov_engine_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(vocab)
+    x = rows_of(kind, n, vocab, g)
+    t, p, k = (torch.tensor([OPTIONS[i % len(OPTIONS)][j] for i in range(n)], device=DEV) for j in range(3))
+    out, probs = torch.empty(n, dtype=torch.int32, device=DEV), torch.empty(n, vocab, device=DEV)
+    seeds = torch.arange(3 * n, device=DEV, dtype=torch.int32).view(n, 3)
+    ops.sample(out, x, t, p, k.int(), seeds, probs_out=probs)
+    for i in range(n):
+        temperature, top_p, top_k = OPTIONS[i % len(OPTIONS)]
+        kept = probs[i] > 0
+        mass = torch.exp((x[i].double() - x[i].double().max()) / temperature)
+        stays = torch.ones_like(kept)
+        if 0 < top_k < vocab:
+            stays = x[i] >= torch.topk(x[i], top_k).values[-1]
+        # kept: nothing but what top-k leaves, whole ties, and down to a value above which lies at most top_p of that mass
+        # (32-bit exponentials of numbers up to 28 and masses in 2^-40 of the largest: some 1e-5; what they round to zero
+        # is not seen in the probabilities)
+        assert not bool((kept & ~stays).any()) and int(out[i]) < vocab and bool(kept[out[i].long()])
+        least = x[i][kept].min()
+        seen = stays & (mass / mass[kept].sum() > 1e-30)
+        assert bool((kept == (seen & (x[i] >= least))).all())
+        if top_p < 1.0:
+            all_mass = mass[stays].sum()
+            assert float(mass[stays & (x[i] > least)].sum()) <= (top_p + 2e-5) * float(all_mass)
+            assert float(mass[stays & (x[i] >= least)].sum()) >= (top_p - 2e-5) * float(all_mass)
+        else:
+            assert bool((kept == seen).all())
