@@ -21,9 +21,11 @@ class Sampler:
         self.max_rows = max_rows
         # A ring of pinned buffers: the copy to the device runs when the device gets to it, which may be after
         # the next call has been made (the engine launches steps ahead of reading their results).
-        self._hosts = [(torch.empty((max_rows, 6), dtype=torch.int32, pin_memory=True), torch.cuda.Event()) for _ in range(4)]
+        # A call's options stand one kind behind the other, as the kernel reads them: n temperatures, n top_p, n top_k,
+        # n triples (seed low word, seed high word, counter).
+        self._hosts = [(torch.empty(max_rows * 6, dtype=torch.int32, pin_memory=True), torch.cuda.Event()) for _ in range(4)]
         self._host_at = 0
-        self._dev = torch.empty((max_rows, 6), dtype=torch.int32, device=device)
+        self._dev = torch.empty(max_rows * 6, dtype=torch.int32, device=device)
         self._out = torch.empty(max_rows, dtype=torch.int32, device=device)
         self._scratch = None
 
@@ -42,22 +44,20 @@ class Sampler:
         pinned, event = self._hosts[self._host_at]
         self._host_at = (self._host_at + 1) % len(self._hosts)
         event.synchronize()
+        # (whole columns at a time: 64 rows value by value took 160 us, and two kernels to turn them into columns)
         host = pinned.numpy()
-        f = host.view(np.float32)
-        for i, p in enumerate(params):
-            f[i, 0] = p.temperature
-            f[i, 1] = p.top_p
-            host[i, 2] = p.top_k
-            seed = int(p.seed) & 0xFFFFFFFFFFFFFFFF
-            host[i, 3:5] = np.array([seed & 0xFFFFFFFF, seed >> 32], dtype=np.uint32).view(np.int32)
-            host[i, 5] = token_indices[i]
-        self._dev[:n].copy_(pinned[:n], non_blocking=True)
+        floats = host.view(np.float32)
+        floats[:n] = [p.temperature for p in params]
+        floats[n:2 * n] = [p.top_p for p in params]
+        host[2 * n:3 * n] = np.array([p.top_k for p in params], dtype=np.int32)
+        triples = host[3 * n:6 * n].reshape(n, 3)
+        seeds = np.array([int(p.seed) & 0xFFFFFFFFFFFFFFFF for p in params], dtype=np.uint64)
+        triples[:, :2] = seeds.view(np.int32).reshape(n, 2)          # (low word first)
+        triples[:, 2] = np.array(token_indices[:n], dtype=np.int32)
+        d = self._dev[:6 * n]
+        d.copy_(pinned[:6 * n], non_blocking=True)
         event.record()
-        d = self._dev[:n]
-        cols = d.t().contiguous()  # [6, n]: each option contiguous
-        temperature = cols[0].view(torch.float32)
-        top_p = cols[1].view(torch.float32)
-        top_k = cols[2]
-        seeds = d[:, 3:6].contiguous()
+        temperature, top_p = d[:2 * n].view(torch.float32).view(2, n)
+        top_k, seeds = d[2 * n:3 * n], d[3 * n:].view(n, 3)
         ops.sample(out, logits, temperature, top_p, top_k, seeds)
         return out
