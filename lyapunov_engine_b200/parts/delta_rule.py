@@ -110,9 +110,12 @@ class GatedDeltaMixer(Mixer):
                                    tile_request, tile_q0, num_tiles, add_input=False, silu=True)
         o = ws.get("delta_out", (T, H * e), torch.float32)
         scratch = ws.get("delta_numbers", (T, ops.gated_delta_scratch_width(H, G)), torch.float32)
+        chunk_scratch = None
+        if not ctx.pure_decode:
+            chunk_scratch = ws.get("delta_chunks", (ops.gated_delta_chunk_floats(T, ctx.num_requests, H),), torch.float32)
         ops.gated_delta_scan(o, conv, self.q_col, self.k_col, self.v_col, proj, self.beta_col, self.decay_col, self.a_log,
                              self.dt_bias, cache.state, ctx.state_slots, ctx.cu_q, ctx.num_requests, H, G, d, e, UNIT_EPS,
-                             d ** -0.5, scratch=scratch)
+                             d ** -0.5, scratch=scratch, chunk_scratch=chunk_scratch)
         gated = ws.get("delta_gated", (T, H * e), rt.dtype)
         ops.head_norm_gate(gated, o, proj[:, self.gate_col:self.gate_col + H * e], self.norm_weight, self.norm_eps, H, e)
         return ops.linear_for_residual(gated, self.w_o, ws, "mixer_out", ctx.status)

@@ -109,12 +109,12 @@ def test_delta_rule_under_every_cut(H, G, d, e, dtype):
 
 
 @pytest.mark.parametrize("H,G,d,e", [(2, 1, 72, 8), (4, 2, 128, 16), (2, 2, 96, 40), (1, 1, 120, 24)])
-def test_delta_rule_in_groups_of_tokens(H, G, d, e):
-    """bfloat16 heads of 65 to 128 entries: portions that end anywhere in a
-    group of four tokens and in a tile of eight, more tiles than the ring has
-    stages, and single tokens among portions."""
+def test_delta_rule_over_chunks(H, G, d, e):
+    """bfloat16 heads of 65 to 128 entries: portions that end at and around the
+    borders of chunks (16 tokens), more chunks than the ring has stages, and
+    single tokens among portions."""
     g = torch.Generator().manual_seed(H * 100 + d)
-    cuts = [[2, 3, 4, 5, 6, 7, 8, 9], [1, 66, 1, 3], [57, 1, 2, 64, 65]]
+    cuts = [[2, 15, 16, 17, 1, 31], [1, 66, 1, 3], [57, 1, 2, 64, 161]]
     a_log, dt_bias = torch.randn(H, generator=g) * 0.5 - 1.0, torch.randn(H, generator=g) * 0.5
     seqs = []
     for n in map(sum, cuts):
@@ -122,7 +122,7 @@ def test_delta_rule_in_groups_of_tokens(H, G, d, e):
         seqs.append(tuple((torch.randn(*shape, generator=g) * f).bfloat16().float() for shape, f in zip(shapes, (1, 3, 1, 2, 2))))
     got, _ = run_delta(seqs, cuts, [2, 0, 3], 5, H, G, d, e, a_log, dt_bias, torch.bfloat16)
     for r in range(3):
-        # 32-bit sums of d products and a state of up to 190 tokens: the bound of the test above
+        # 32-bit sums of d products and a state of up to 285 tokens: the bound of the test above
         torch.testing.assert_close(got[r], plain_delta(*seqs[r], a_log, dt_bias, H, G, d, e).float(), atol=3e-5, rtol=3e-5)
 
 
