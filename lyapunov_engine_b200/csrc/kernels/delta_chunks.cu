@@ -38,7 +38,7 @@
 namespace {
 
 using bf16 = __nv_bfloat16;
-using le::add4, le::ldsm4, le::ldsm4_trans, le::mma, le::mma_first, le::mma_split3, le::split_pair3;
+using le::ldsm4, le::ldsm4_trans, le::mma, le::mma_first, le::mma_split3, le::split_pair3;
 
 constexpr int CHUNK = 16;
 constexpr int DIM = 128;                    // entries of a head, padded
@@ -60,6 +60,7 @@ struct DeltaArgs {
   const float *a_log, *dt_bias;
   float *state; int num_state_rows;
   const int32_t *state_slots, *cu_q;
+  const int32_t *requests;                  // the requests this launch takes, or null: all in order
   int heads, kv_heads, dim, vdim;
   float unit_eps, q_scale;
   float *numbers;                           // [tokens / 16 + requests, heads, NUMBERS]
@@ -72,7 +73,7 @@ delta_chunk_numbers_kernel(DeltaArgs p) {
   __shared__ __align__(16) float s_k[CHUNK][LDF], s_q[CHUNK][LDF];
   __shared__ float s_inv[2][CHUNK], s_g[CHUNK], s_beta[CHUNK], s_a[CHUNK][CHUNK + 1], s_x[CHUNK][CHUNK + 1], s_p[CHUNK][CHUNK + 1];
   le::let_successor_start();
-  const int group = blockIdx.y, b = blockIdx.z;
+  const int group = blockIdx.y, b = p.requests != nullptr ? p.requests[blockIdx.z] : blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int i = tid / CHUNK, j = tid % CHUNK;
   const int first = p.cu_q[b], q_len = p.cu_q[b + 1] - first;
@@ -179,7 +180,7 @@ delta_chunk_kernel(DeltaArgs p) {
   Meeting &meet = *reinterpret_cast<Meeting *>(delta_smem);
   Stage *ring = reinterpret_cast<Stage *>(delta_smem + sizeof(Meeting));
   le::let_successor_start();
-  const int b = blockIdx.z, h = blockIdx.y, e0 = blockIdx.x * COLS;
+  const int b = p.requests != nullptr ? p.requests[blockIdx.z] : blockIdx.z, h = blockIdx.y, e0 = blockIdx.x * COLS;
   const int first = p.cu_q[b], q_len = p.cu_q[b + 1] - first;
   const int slot = p.state_slots[b];
   const bool kept = slot >= 0 && slot < p.num_state_rows;
@@ -326,7 +327,7 @@ int launch_walk(const DeltaArgs &p, dim3 grid, size_t least, cudaStream_t stream
 }  // namespace
 
 // The scratch of le_gated_delta_chunks: tokens / le_gated_delta_chunk() + requests rows of le_gated_delta_chunk_width()
-// floats.
+// floats (the step's tokens and requests, those that are not listed too).
 LE_API int le_gated_delta_chunk() { return CHUNK; }
 LE_API int le_gated_delta_chunk_width(int heads) { return heads * NUMBERS; }
 
@@ -340,13 +341,15 @@ LE_API int le_gated_delta_chunks_apply(const void *qkv, int64_t qkv_stride, int 
              : 0;
 }
 
-// le_gated_delta_scan's recurrence over chunks, where le_gated_delta_chunks_apply.  scratch:
-// (see le_gated_delta_chunk_width), 16-byte aligned.
+// le_gated_delta_scan's recurrence over chunks, where le_gated_delta_chunks_apply.  requests: the indices of the
+// num_requests requests to run, or null: requests 0 .. num_requests - 1; num_tokens: their tokens in all (it only
+// chooses the launch's shape).  scratch: see le_gated_delta_chunk_width, 16-byte aligned.
 LE_API int le_gated_delta_chunks(float *out, int64_t out_stride, const void *qkv, int64_t qkv_stride, int q_col, int k_col,
                                  int v_col, const void *proj, int64_t proj_stride, int b_col, int a_col, const float *a_log,
                                  const float *dt_bias, float *state, int num_state_rows, const int32_t *state_slots,
-                                 const int32_t *cu_q, int num_requests, int num_tokens, int heads, int kv_heads, int dim,
-                                 int vdim, float unit_eps, float q_scale, float *scratch, cudaStream_t stream) {
+                                 const int32_t *cu_q, const int32_t *requests, int num_requests, int num_tokens, int heads,
+                                 int kv_heads, int dim, int vdim, float unit_eps, float q_scale, float *scratch,
+                                 cudaStream_t stream) {
   if (num_requests <= 0 || num_tokens <= 0) return 0;
   if (heads < 1 || kv_heads < 1 || heads % kv_heads) return le::invalid("le_gated_delta_chunks: %d heads, %d groups", heads, kv_heads);
   if (!le_gated_delta_chunks_apply(qkv, qkv_stride, q_col, k_col, v_col, LE_BF16, dim, vdim) ||
@@ -356,7 +359,7 @@ LE_API int le_gated_delta_chunks(float *out, int64_t out_stride, const void *qkv
   p.out = out, p.out_stride = out_stride, p.qkv = static_cast<const bf16 *>(qkv), p.qkv_stride = qkv_stride;
   p.q_col = q_col, p.k_col = k_col, p.v_col = v_col, p.proj = static_cast<const bf16 *>(proj), p.proj_stride = proj_stride;
   p.b_col = b_col, p.a_col = a_col, p.a_log = a_log, p.dt_bias = dt_bias, p.state = state, p.num_state_rows = num_state_rows;
-  p.state_slots = state_slots, p.cu_q = cu_q, p.heads = heads, p.kv_heads = kv_heads, p.dim = dim, p.vdim = vdim;
+  p.state_slots = state_slots, p.cu_q = cu_q, p.requests = requests, p.heads = heads, p.kv_heads = kv_heads, p.dim = dim, p.vdim = vdim;
   p.unit_eps = unit_eps, p.q_scale = q_scale, p.numbers = scratch;
   const int most = (num_tokens + CHUNK - 1) / CHUNK;    // chunks of one request, if it has all the tokens
   const dim3 grid((vdim + COLS - 1) / COLS, heads, num_requests);

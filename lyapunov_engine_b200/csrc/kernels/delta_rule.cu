@@ -35,8 +35,9 @@
 // Rows that stand for no request (slot < 0) give zeros and keep nothing.  In a
 // step of single tokens the block has no fetching warps.
 //
-// Prompts in bfloat16 with heads of 65 to 128 entries go over chunks on the
-// tensor cores instead (delta_chunks.cu).
+// Requests with several tokens in bfloat16, heads of 65 to 128 entries, have a
+// form over chunks on the tensor cores (delta_chunks.cu); the scan then takes the
+// decoded tokens beside them, a list of requests.
 //
 // head_norm_gate_kernel: o of every (token, head) is divided by its root mean
 // square over vdim, times a weight ([vdim], the same for every head, or [heads,
@@ -65,38 +66,43 @@ template <typename T>
 __global__ void __launch_bounds__(PREP_THREADS)
 gated_delta_prepare_kernel(float *__restrict__ prep, int prep_stride, const T *__restrict__ qkv, int64_t qkv_stride, int q_col,
                            int k_col, const T *__restrict__ proj, int64_t proj_stride, int b_col, int a_col,
-                           const float *__restrict__ a_log, const float *__restrict__ dt_bias, int heads, int kv_heads,
+                           const float *__restrict__ a_log, const float *__restrict__ dt_bias,
+                           const int32_t *__restrict__ cu_q, const int32_t *__restrict__ requests, int heads, int kv_heads,
                            int dim, float unit_eps, float q_scale) {
   le::let_successor_start();
+  // a block takes a token, or, of listed requests, all of one
+  const int64_t t_begin = requests != nullptr ? cu_q[requests[blockIdx.x]] : blockIdx.x;
+  const int64_t t_end = requests != nullptr ? cu_q[requests[blockIdx.x] + 1] : t_begin + 1;
   le::wait_for_predecessor();
-  const int64_t t = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = PREP_THREADS / 32;
-  float *dst = prep + t * prep_stride;
-  for (int g = blockIdx.y * warps + warp; g < kv_heads; g += gridDim.y * warps) {
-    const T *kr = qkv + t * qkv_stride + k_col + g * dim;
-    const T *qr = qkv + t * qkv_stride + q_col + g * dim;
-    float kk = 0.0f, qq = 0.0f, kq = 0.0f;
-    for (int i = lane; i < dim; i += 32) {
-      const float a = le::to_f32(kr[i]), c = le::to_f32(qr[i]);
-      kk = fmaf(a, a, kk);
-      qq = fmaf(c, c, qq);
-      kq = fmaf(a, c, kq);
+  for (int64_t t = t_begin; t < t_end; ++t) {
+    float *dst = prep + t * prep_stride;
+    for (int g = blockIdx.y * warps + warp; g < kv_heads; g += gridDim.y * warps) {
+      const T *kr = qkv + t * qkv_stride + k_col + g * dim;
+      const T *qr = qkv + t * qkv_stride + q_col + g * dim;
+      float kk = 0.0f, qq = 0.0f, kq = 0.0f;
+      for (int i = lane; i < dim; i += 32) {
+        const float a = le::to_f32(kr[i]), c = le::to_f32(qr[i]);
+        kk = fmaf(a, a, kk);
+        qq = fmaf(c, c, qq);
+        kq = fmaf(a, c, kq);
+      }
+      kk = le::warp_sum(kk);
+      qq = le::warp_sum(qq);
+      kq = le::warp_sum(kq);
+      if (lane == 0) {
+        const float k_inv = rsqrtf(kk + unit_eps), q_inv = rsqrtf(qq + unit_eps) * q_scale;
+        dst[4 * g + 0] = k_inv;
+        dst[4 * g + 1] = q_inv;
+        dst[4 * g + 2] = kq * k_inv * q_inv;
+        dst[4 * g + 3] = 0.0f;
+      }
     }
-    kk = le::warp_sum(kk);
-    qq = le::warp_sum(qq);
-    kq = le::warp_sum(kq);
-    if (lane == 0) {
-      const float k_inv = rsqrtf(kk + unit_eps), q_inv = rsqrtf(qq + unit_eps) * q_scale;
-      dst[4 * g + 0] = k_inv;
-      dst[4 * g + 1] = q_inv;
-      dst[4 * g + 2] = kq * k_inv * q_inv;
-      dst[4 * g + 3] = 0.0f;
+    for (int h = blockIdx.y * PREP_THREADS + threadIdx.x; h < heads; h += gridDim.y * PREP_THREADS) {
+      const float av = le::to_f32(proj[t * proj_stride + a_col + h]), bv = le::to_f32(proj[t * proj_stride + b_col + h]);
+      dst[4 * kv_heads + 2 * h + 0] = expf(-expf(a_log[h]) * softplus_f32(av + dt_bias[h]));
+      dst[4 * kv_heads + 2 * h + 1] = sigmoid_f32(bv);
     }
-  }
-  for (int h = blockIdx.y * PREP_THREADS + threadIdx.x; h < heads; h += gridDim.y * PREP_THREADS) {
-    const float av = le::to_f32(proj[t * proj_stride + a_col + h]), bv = le::to_f32(proj[t * proj_stride + b_col + h]);
-    dst[4 * kv_heads + 2 * h + 0] = expf(-expf(a_log[h]) * softplus_f32(av + dt_bias[h]));
-    dst[4 * kv_heads + 2 * h + 1] = sigmoid_f32(bv);
   }
 }
 
@@ -167,7 +173,7 @@ __global__ void __launch_bounds__(SCAN_THREADS)
 gated_delta_scan_kernel(float *__restrict__ out, int64_t out_stride, const T *__restrict__ qkv, int64_t qkv_stride, int q_col,
                         int k_col, int v_col, const float *__restrict__ prep, int prep_stride, float *__restrict__ state,
                         int num_state_rows, const int32_t *__restrict__ state_slots, const int32_t *__restrict__ cu_q,
-                        int heads, int kv_heads, int dim, int vdim, int tile, int wide) {
+                        const int32_t *__restrict__ requests, int heads, int kv_heads, int dim, int vdim, int tile, int wide) {
   extern __shared__ __align__(16) unsigned char scan_smem[];
   constexpr int QUADS = ROWS / 4;                   // groups of four rows a thread holds
   constexpr int DPAD = ROWS * LANES;
@@ -177,7 +183,7 @@ gated_delta_scan_kernel(float *__restrict__ out, int64_t out_stride, const T *__
   const int buf_floats = 2 * vec_floats + tile * (COLS + SCAN_NUMBERS);
   float *smem = reinterpret_cast<float *>(scan_smem);
   le::let_successor_start();
-  const int b = blockIdx.z, h = blockIdx.y;
+  const int b = requests != nullptr ? requests[blockIdx.z] : blockIdx.z, h = blockIdx.y;
   const int group = h / (heads / kv_heads);
   const int first = cu_q[b], q_len = cu_q[b + 1] - first;
   const int slot = state_slots[b];
@@ -440,13 +446,15 @@ LE_API int le_gated_delta_scratch(int heads, int kv_heads) { return 4 * kv_heads
 // out [tokens, heads * vdim] float32.  qkv: rows holding the convolved, activated queries and keys [kv_heads, dim]
 // at columns q_col and k_col and values [heads, vdim] at v_col.  proj: rows holding one number per head at b_col
 // (step size before its sigmoid) and at a_col (decay before its softplus).  state: [rows, heads, vdim, dim] float32.
-// scratch: [tokens, le_gated_delta_scratch()] float32, rewritten here.
+// requests: the indices of the num_requests requests to run, or null: requests 0 .. num_requests - 1; num_tokens: their
+// tokens in all (listed requests: it only chooses the launch's shape).
+// scratch: [tokens of the step, le_gated_delta_scratch()] float32, rewritten here.
 LE_API int le_gated_delta_scan(float *out, int64_t out_stride, const void *qkv, int64_t qkv_stride, int q_col, int k_col,
                                int v_col, const void *proj, int64_t proj_stride, int b_col, int a_col, int dtype,
                                const float *a_log, const float *dt_bias, float *state, int num_state_rows,
-                               const int32_t *state_slots, const int32_t *cu_q, int num_requests, int num_tokens, int heads,
-                               int kv_heads, int dim, int vdim, float unit_eps, float q_scale, float *scratch,
-                               cudaStream_t stream) {
+                               const int32_t *state_slots, const int32_t *cu_q, const int32_t *requests, int num_requests,
+                               int num_tokens, int heads, int kv_heads, int dim, int vdim, float unit_eps, float q_scale,
+                               float *scratch, cudaStream_t stream) {
   if (num_requests <= 0 || num_tokens <= 0) return 0;
   if (heads < 1 || kv_heads < 1 || heads % kv_heads) return le::invalid("le_gated_delta_scan: %d heads, %d groups", heads, kv_heads);
   int rows = 0, lanes = 0;
@@ -465,7 +473,7 @@ LE_API int le_gated_delta_scan(float *out, int64_t out_stride, const void *qkv, 
   if (single) tile = 1;
   const int threads = single ? SCAN_HOLDERS : SCAN_THREADS;
   const size_t smem = 2 * tile * per_token;
-  const dim3 prep_grid(num_tokens, (kv_heads + PREP_THREADS / 32 - 1) / (PREP_THREADS / 32));
+  const dim3 prep_grid(requests != nullptr ? num_requests : num_tokens, (kv_heads + PREP_THREADS / 32 - 1) / (PREP_THREADS / 32));
   const dim3 grid((vdim + cols - 1) / cols, heads, num_requests);
   if (grid.y > 65535 || grid.z > 65535 || prep_grid.y > 65535)
     return le::invalid("le_gated_delta_scan: too many heads or requests for one launch");
@@ -473,15 +481,15 @@ LE_API int le_gated_delta_scan(float *out, int64_t out_stride, const void *qkv, 
   do {                                                                                                                  \
     int rc = le::launch_chained(gated_delta_prepare_kernel<T>, prep_grid, dim3(PREP_THREADS), 0, stream, scratch,       \
                                 prep_stride, static_cast<const T *>(qkv), qkv_stride, q_col, k_col,                     \
-                                static_cast<const T *>(proj), proj_stride, b_col, a_col, a_log, dt_bias, heads, kv_heads, \
-                                dim, unit_eps, q_scale);                                                                \
+                                static_cast<const T *>(proj), proj_stride, b_col, a_col, a_log, dt_bias, cu_q, requests,   \
+                                heads, kv_heads, dim, unit_eps, q_scale);                                                                \
     if (rc != 0) return rc;                                                                                             \
     if (smem > 48 * 1024)                                                                                               \
       cudaFuncSetAttribute(gated_delta_scan_kernel<T, R, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
     return le::launch_chained(gated_delta_scan_kernel<T, R, L>, grid, dim3(threads), smem, stream, out, out_stride,     \
                               static_cast<const T *>(qkv), qkv_stride, q_col, k_col, v_col,                             \
                               static_cast<const float *>(scratch), prep_stride, state, num_state_rows, state_slots, cu_q, \
-                              heads, kv_heads, dim, vdim, tile, wide);                                                  \
+                              requests, heads, kv_heads, dim, vdim, tile, wide);                                                  \
   } while (0)
 #define LE_SHAPE(T, R, L) \
   if (rows == R && lanes == L) LE_GO(T, R, L)

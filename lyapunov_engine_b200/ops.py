@@ -88,12 +88,12 @@ _CORE_SIGNATURES = {
     "le_gated_delta_chunk_width": [c_int],
     "le_gated_delta_chunks_apply": [c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int, c_int],
     "le_gated_delta_chunks": [c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_void_p, c_int64, c_int, c_int, c_void_p,
-                              c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
-                              c_float, c_void_p, c_void_p],
+                              c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
+                              c_float, c_float, c_void_p, c_void_p],
     "le_gated_delta_scratch": [c_int, c_int],
     "le_gated_delta_scan": [c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_void_p, c_int64, c_int, c_int, c_int,
-                            c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
-                            c_float, c_float, c_void_p, c_void_p],
+                            c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+                            c_int, c_float, c_float, c_void_p, c_void_p],
     "le_head_norm_gate": [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_void_p, c_float, c_int, c_int,
                           c_int, c_int, c_int, c_float, c_void_p],
     "le_rope_norm_store": [c_void_p, c_int64, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int,
@@ -1375,53 +1375,70 @@ def gated_delta_scratch_width(heads: int, kv_heads: int) -> int:
     return 4 * int(kv_heads) + 2 * int(heads)
 
 
-def gated_delta_chunk_floats(num_tokens: int, num_requests: int, heads: int) -> int:
-    """Floats of ``chunk_scratch`` for ``gated_delta_scan``."""
-    return (int(num_tokens) // core().le_gated_delta_chunk() + int(num_requests)) * core().le_gated_delta_chunk_width(int(heads))
-
-
-def gated_delta_scan(out, qkv, q_col, k_col, v_col, proj, b_col, a_col, a_log, dt_bias, state, state_slots, cu_q,
-                     num_requests, heads, kv_heads, dim, vdim, unit_eps, q_scale, scratch=None, chunk_scratch=None) -> None:
-    """The gated delta rule over the step's tokens, request by request, from
-    each request's state row and back into it.  ``out``: float32 [T, heads *
-    vdim].  ``qkv``: rows with queries and keys [kv_heads, dim] at columns
-    ``q_col`` / ``k_col`` and values [heads, vdim] at ``v_col``; queries and
-    keys are made unit vectors here (x / sqrt(sum x^2 + unit_eps)), queries
-    times ``q_scale``.  ``proj``: rows with one number per head at ``b_col``
-    (step size = its sigmoid) and ``a_col`` (decay = exp(-exp(a_log) *
-    softplus(a + dt_bias))).  ``state``: float32 [rows, heads, vdim, dim].
-    ``scratch``: float32 [T, gated_delta_scratch_width()], made here if None.
-    A step with more tokens than requests runs over chunks on the tensor cores
-    where that form applies (bfloat16, heads of 65 to 128 entries, rows of
-    whole 16-byte pieces); ``chunk_scratch``: float32, at least
-    gated_delta_chunk_floats(), made here if None."""
-    _need_cuda(out, qkv, proj, a_log, dt_bias, state, state_slots, cu_q)
+def _gated_delta_checks(out, qkv, proj, a_log, dt_bias, state, heads, dim, vdim) -> None:
     T = out.shape[0]
     assert out.dtype == torch.float32 and out.stride(1) == 1 and qkv.stride(1) == 1 and proj.stride(1) == 1
     assert qkv.dtype == proj.dtype and a_log.dtype == torch.float32 and dt_bias.dtype == torch.float32
     assert a_log.numel() == heads and dt_bias.numel() == heads and qkv.shape[0] == T and proj.shape[0] == T
     assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (heads, vdim, dim)
-    if T > num_requests and core().le_gated_delta_chunks_apply(_ptr(qkv), qkv.stride(0), q_col, k_col, v_col, dtype_code(qkv.dtype),
-                                                               dim, vdim) and state.data_ptr() % 16 == 0:
-        floats = gated_delta_chunk_floats(T, num_requests, heads)
-        if chunk_scratch is None:
-            chunk_scratch = torch.empty(floats, dtype=torch.float32, device=out.device)
-        assert chunk_scratch.dtype == torch.float32 and chunk_scratch.is_contiguous() and chunk_scratch.numel() >= floats
-        _check(core().le_gated_delta_chunks(_ptr(out), out.stride(0), _ptr(qkv), qkv.stride(0), q_col, k_col, v_col, _ptr(proj),
-                                            proj.stride(0), b_col, a_col, _ptr(a_log), _ptr(dt_bias), _ptr(state), state.shape[0],
-                                            _ptr(state_slots), _ptr(cu_q), num_requests, T, heads, kv_heads, dim, vdim,
-                                            float(unit_eps), float(q_scale), _ptr(chunk_scratch), _stream()),
-               "le_gated_delta_chunks", launches=2)
-        return
+
+
+def gated_delta_scan(out, qkv, q_col, k_col, v_col, proj, b_col, a_col, a_log, dt_bias, state, state_slots, cu_q,
+                     num_requests, heads, kv_heads, dim, vdim, unit_eps, q_scale, scratch=None, requests=None) -> None:
+    """The gated delta rule over the step's tokens, request by request, from
+    each request's state row and back into it.  ``out``: float32 [T, heads *
+    vdim].  ``qkv``: rows with queries and keys [kv_heads, dim] at columns
+    ``q_col`` and ``k_col`` and values [heads, vdim] at ``v_col``; queries and
+    keys are made unit vectors here (``unit_eps`` under the root), queries
+    times ``q_scale``.  ``proj``: rows with one number per head at ``b_col``
+    (step size = its sigmoid) and ``a_col`` (decay = exp(-exp(a_log) *
+    softplus(a + dt_bias))).  ``state``: float32 [rows, heads, vdim, dim].
+    ``scratch``: float32 [T, gated_delta_scratch_width()], made here if None.
+    ``requests``: int32 indices of the ``num_requests`` requests to run (None:
+    the first ones)."""
+    _need_cuda(out, qkv, proj, a_log, dt_bias, state, state_slots, cu_q, scratch, requests)
+    _gated_delta_checks(out, qkv, proj, a_log, dt_bias, state, heads, dim, vdim)
+    T = out.shape[0]
     width = gated_delta_scratch_width(heads, kv_heads)
     if scratch is None:
         scratch = torch.empty((max(T, 1), width), dtype=torch.float32, device=out.device)
     assert scratch.dtype == torch.float32 and scratch.is_contiguous() and scratch.shape[0] >= T and scratch.shape[1] == width
     _check(core().le_gated_delta_scan(_ptr(out), out.stride(0), _ptr(qkv), qkv.stride(0), q_col, k_col, v_col, _ptr(proj),
                                       proj.stride(0), b_col, a_col, dtype_code(qkv.dtype), _ptr(a_log), _ptr(dt_bias),
-                                      _ptr(state), state.shape[0], _ptr(state_slots), _ptr(cu_q), num_requests, T, heads,
-                                      kv_heads, dim, vdim, float(unit_eps), float(q_scale), _ptr(scratch), _stream()),
+                                      _ptr(state), state.shape[0], _ptr(state_slots), _ptr(cu_q), _ptr(requests), num_requests,
+                                      T if requests is None else num_requests, heads, kv_heads, dim, vdim, float(unit_eps),
+                                      float(q_scale), _ptr(scratch), _stream()),
            "le_gated_delta_scan")
+
+
+def gated_delta_chunks_apply(dtype, row_stride: int, q_col: int, k_col: int, v_col: int, dim: int, vdim: int) -> bool:
+    """Whether gated_delta_chunks() takes rows of this type, pitch and columns
+    (on a 16-byte address) and heads of these sizes."""
+    return bool(core().le_gated_delta_chunks_apply(None, row_stride, q_col, k_col, v_col, dtype_code(dtype), dim, vdim))
+
+
+def gated_delta_chunk_floats(num_tokens: int, num_requests: int, heads: int) -> int:
+    """Floats of ``scratch`` for gated_delta_chunks() in a step of so many tokens and requests."""
+    return (int(num_tokens) // core().le_gated_delta_chunk() + int(num_requests)) * core().le_gated_delta_chunk_width(int(heads))
+
+
+def gated_delta_chunks(out, qkv, q_col, k_col, v_col, proj, b_col, a_col, a_log, dt_bias, state, state_slots, cu_q, requests,
+                       num_requests, heads, kv_heads, dim, vdim, unit_eps, q_scale, scratch) -> None:
+    """gated_delta_scan() over chunks of tokens on the tensor cores for the
+    ``num_requests`` requests that ``requests`` (int32 indices) lists, where
+    gated_delta_chunks_apply().  ``scratch``: float32, 16-byte aligned,
+    gated_delta_chunk_floats() of the whole step."""
+    _need_cuda(out, qkv, proj, a_log, dt_bias, state, state_slots, cu_q, requests, scratch)
+    _gated_delta_checks(out, qkv, proj, a_log, dt_bias, state, heads, dim, vdim)
+    T = out.shape[0]
+    assert qkv.dtype == torch.bfloat16 and requests.dtype == torch.int32 and requests.numel() >= num_requests
+    assert scratch.dtype == torch.float32 and scratch.is_contiguous()
+    assert scratch.numel() >= gated_delta_chunk_floats(T, cu_q.numel() - 1, heads)
+    _check(core().le_gated_delta_chunks(_ptr(out), out.stride(0), _ptr(qkv), qkv.stride(0), q_col, k_col, v_col, _ptr(proj),
+                                        proj.stride(0), b_col, a_col, _ptr(a_log), _ptr(dt_bias), _ptr(state), state.shape[0],
+                                        _ptr(state_slots), _ptr(cu_q), _ptr(requests), num_requests, T, heads, kv_heads, dim,
+                                        vdim, float(unit_eps), float(q_scale), _ptr(scratch), _stream()),
+           "le_gated_delta_chunks", launches=2)
 
 
 def head_norm_gate(out, o, gate, weight, eps, heads, vdim, sigmoid: bool = False, out_scale: float = 1.0) -> None:

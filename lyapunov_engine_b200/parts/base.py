@@ -184,6 +184,10 @@ class PositionEncoding(Part):
         raise NotImplementedError
 
 
+# A tile size beyond any request's tokens: ctx.tiles[WHOLE] lists a step's requests, those with several tokens first.
+WHOLE = 1 << 30
+
+
 class Mixer(Part):
     # a bias [H] (32-bit) on the output that forward() leaves to the block that adds the output to the stream (named
     # by ``o_bias_name``; blocks that add none refuse such a mixer)

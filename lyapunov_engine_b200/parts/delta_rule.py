@@ -16,7 +16,9 @@ S [d, e] starts at zero and is carried from token to token in 32 bits, one
 matrix per request and head (``state_need``); the convolutions' last taps - 1
 inputs are state of the request too (``extra_state_needs``).  One product makes
 all six projections; the convolution, the recurrence and the gated norm are a
-kernel each (ops.short_conv_general, ops.gated_delta_scan, ops.head_norm_gate).
+kernel each (ops.short_conv_general, ops.gated_delta_scan, ops.head_norm_gate);
+requests that bring several tokens in bfloat16, heads of 65 to 128 entries, go
+over chunks on the tensor cores (ops.gated_delta_chunks).
 Unit vectors, decays, step sizes, the recurrence and the norm are 32-bit.
 """
 from __future__ import annotations
@@ -24,7 +26,7 @@ from __future__ import annotations
 import torch
 
 from .. import ops
-from .base import Mixer, StateNeed, TensorDecl, register_mixer
+from .base import WHOLE, Mixer, StateNeed, TensorDecl, register_mixer
 
 UNIT_EPS = 1e-6
 
@@ -65,7 +67,7 @@ class GatedDeltaMixer(Mixer):
         return {"mixer_taps": StateNeed((self.taps - 1, self.channels), torch.float32)}
 
     def tile_sizes(self):
-        return [ops.SHORT_CONV_TILE]
+        return [ops.SHORT_CONV_TILE, WHOLE]
 
     def tensors(self):
         q, k, v, gate, beta, decay = self.names
@@ -90,6 +92,8 @@ class GatedDeltaMixer(Mixer):
         self.w_taps = torch.cat([get(n + self.conv_suffix) for n in (q, k, v)], dim=0).t().contiguous()   # [taps, channels]
         self.w_o = get(self.o_name)
         self.a_log, self.dt_bias, self.norm_weight = get(self.a_log_name), get(self.dt_bias_name), get(self.norm_name)
+        self.chunks = ops.gated_delta_chunks_apply(runtime.dtype, self.channels, self.q_col, self.k_col, self.v_col, self.head_dim,
+                                                   self.value_dim)
         self.runtime = runtime
 
     def forward(self, x, ctx, cache):
@@ -109,13 +113,20 @@ class GatedDeltaMixer(Mixer):
             ops.short_conv_general(conv, proj[:, :self.channels], self.w_taps, taps_state, ctx.state_slots, ctx.cu_q,
                                    tile_request, tile_q0, num_tiles, add_input=False, silu=True)
         o = ws.get("delta_out", (T, H * e), torch.float32)
-        scratch = ws.get("delta_numbers", (T, ops.gated_delta_scratch_width(H, G)), torch.float32)
-        chunk_scratch = None
-        if not ctx.pure_decode:
-            chunk_scratch = ws.get("delta_chunks", (ops.gated_delta_chunk_floats(T, ctx.num_requests, H),), torch.float32)
-        ops.gated_delta_scan(o, conv, self.q_col, self.k_col, self.v_col, proj, self.beta_col, self.decay_col, self.a_log,
-                             self.dt_bias, cache.state, ctx.state_slots, ctx.cu_q, ctx.num_requests, H, G, d, e, UNIT_EPS,
-                             d ** -0.5, scratch=scratch, chunk_scratch=chunk_scratch)
+        rows = (o, conv, self.q_col, self.k_col, self.v_col, proj, self.beta_col, self.decay_col, self.a_log, self.dt_bias,
+                cache.state, ctx.state_slots, ctx.cu_q)
+        sizes = (H, G, d, e, UNIT_EPS, d ** -0.5)
+        request, _, _, several = ctx.tiles[WHOLE]
+        if several and self.chunks:
+            numbers = ws.get("delta_chunks", (ops.gated_delta_chunk_floats(T, ctx.num_requests, H),), torch.float32)
+            ops.gated_delta_chunks(*rows, request, several, *sizes, numbers)
+        # decoded tokens keep the scan, whatever stands beside them in the step
+        if not (several and self.chunks) or ctx.num_decode:
+            scratch = ws.get("delta_numbers", (T, ops.gated_delta_scratch_width(H, G)), torch.float32)
+            if several and self.chunks:
+                ops.gated_delta_scan(*rows, ctx.num_decode, *sizes, scratch=scratch, requests=ctx.decode_requests)
+            else:
+                ops.gated_delta_scan(*rows, ctx.num_requests, *sizes, scratch=scratch)
         gated = ws.get("delta_gated", (T, H * e), rt.dtype)
         ops.head_norm_gate(gated, o, proj[:, self.gate_col:self.gate_col + H * e], self.norm_weight, self.norm_eps, H, e)
         return ops.linear_for_residual(gated, self.w_o, ws, "mixer_out", ctx.status)

@@ -46,9 +46,10 @@ def plain_delta(q, k, v, a, b, a_log, dt_bias, H, G, d, e):
                         for j in range(H)], dim=1)
 
 
-def run_delta(seqs, cuts, slots_of, state_rows, H, G, d, e, a_log, dt_bias, dtype, stale=7.0):
+def run_delta(seqs, cuts, slots_of, state_rows, H, G, d, e, a_log, dt_bias, dtype, stale=7.0, chunks=False):
     """Feeds every sequence (q, k, v, a, b) in its cuts, the live requests of a
-    step as one batch, from state rows that hold ``stale`` numbers."""
+    step as one batch, from state rows that hold ``stale`` numbers.
+    ``chunks``: portions over chunks, single tokens through the scan."""
     from lyapunov_engine_b200 import ops
     C = 2 * G * d + H * e
     state = torch.full((state_rows, H, e, d), stale, device=DEV)
@@ -71,8 +72,16 @@ def run_delta(seqs, cuts, slots_of, state_rows, H, G, d, e, a_log, dt_bias, dtyp
         slots = i32(slots_of[r] for r in live)
         ops.zero_fresh_state(state, slots, i32(at[r] for r in live), len(live))
         out = torch.full((qkv.shape[0], H * e), 5.0, device=DEV)
-        ops.gated_delta_scan(out, qkv, 0, G * d, 2 * G * d, ab, 3, 3 + H, a_log.to(DEV), dt_bias.to(DEV), state, slots, cu,
-                             len(live), H, G, d, e, 1e-6, d ** -0.5)
+        many, single = ([b for b, n in enumerate(q_lens) if (n > 1) == several] for several in (True, False))
+        rows = (out, qkv, 0, G * d, 2 * G * d, ab, 3, 3 + H, a_log.to(DEV), dt_bias.to(DEV), state, slots, cu)
+        sizes = (H, G, d, e, 1e-6, d ** -0.5)
+        if not (chunks and many):
+            ops.gated_delta_scan(*rows, len(live), *sizes)
+        else:
+            scratch = torch.empty(ops.gated_delta_chunk_floats(len(qkv), len(live), H), device=DEV)
+            ops.gated_delta_chunks(*rows, i32(many), len(many), *sizes, scratch)
+            if single:
+                ops.gated_delta_scan(*rows, len(single), *sizes, requests=i32(single))
         o = 0
         for r, n in zip(live, q_lens):
             got[r].append(out[o:o + n].cpu().view(n, H, e))
@@ -120,7 +129,7 @@ def test_delta_rule_over_chunks(H, G, d, e):
     for n in map(sum, cuts):
         shapes = ((n, G, d), (n, G, d), (n, H, e), (n, H), (n, H))
         seqs.append(tuple((torch.randn(*shape, generator=g) * f).bfloat16().float() for shape, f in zip(shapes, (1, 3, 1, 2, 2))))
-    got, _ = run_delta(seqs, cuts, [2, 0, 3], 5, H, G, d, e, a_log, dt_bias, torch.bfloat16)
+    got, _ = run_delta(seqs, cuts, [2, 0, 3], 5, H, G, d, e, a_log, dt_bias, torch.bfloat16, chunks=True)
     for r in range(3):
         # 32-bit sums of d products and a state of up to 285 tokens: the bound of the test above
         torch.testing.assert_close(got[r], plain_delta(*seqs[r], a_log, dt_bias, H, G, d, e).float(), atol=3e-5, rtol=3e-5)
