@@ -229,6 +229,7 @@ decay_chunk_kernel(DecayArgs p) {
   float *s_in = s_to + CHUNK, *s_out = s_in + CHUNK, *s_over = s_out + CHUNK;      // s_over [4][4]
   float *s_floor = s_over + 16, *s_row = s_floor + CHUNK, *s_den = s_row + CHUNK;
   float *s_n = s_den + CHUNK;                              // [DP]
+  int *s_bad = reinterpret_cast<int *>(s_out);             // [COLS]: the first token with NaN or infinity, once s_out is used
   le::let_successor_start();
   const int slices = (p.vdim + COLS - 1) / COLS;
   const int head = blockIdx.x / slices, e0 = (blockIdx.x % slices) * COLS;
@@ -426,6 +427,7 @@ decay_chunk_kernel(DecayArgs p) {
       }
     }
     // the state behind the chunk (tokens beyond it have weight zero)
+    uint32_t odd = 0;                                      // a NaN or an infinity among this warp's values
     if (mine) {
 #pragma unroll
       for (int i = 0; i < NT; ++i) S[i][0] *= keep, S[i][1] *= keep, S[i][2] *= keep, S[i][3] *= keep;
@@ -439,6 +441,7 @@ decay_chunk_kernel(DecayArgs p) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const float2 f = u < 2 ? f0 : f1;
+          odd |= (va[u] & 0x7f807f80u) + 0x00800080u;      // (bits 15 and 31: all bits of an exponent)
           split_pair3(low_of(va[u]) * f.x, high_of(va[u]) * f.y, a[0][u], a[1][u], a[2][u]);
         }
 #pragma unroll
@@ -455,7 +458,9 @@ decay_chunk_kernel(DecayArgs p) {
 #pragma unroll 8
       for (int t = 0; t < CHUNK; ++t) n_mine = fmaf(s_to[t], __bfloat162float(s_k[t * LD + tid]), n_mine);
     }
-    __syncthreads();                                       // the weighted scores are there; k and q are used
+    bool poisoned = false;
+    if constexpr (SUMS) __syncthreads();                   // k is used
+    else poisoned = __syncthreads_or((odd & 0x80008000u) != 0);   // the weighted scores are there; k and q are used
     if (c0 + CHUNK < tokens) {
       fetch_k(c0 + CHUNK);
       if constexpr (!SUMS) fetch_q(c0 + CHUNK);
@@ -466,6 +471,19 @@ decay_chunk_kernel(DecayArgs p) {
           const int t = tid >> 1;
           s_den[t] = fmaxf(fabsf(p.q_scale * fmaf(s_from[t], nq, s_row[t])), s_floor[t]) + 1e-6f;
         }
+      }
+      // The weights of keys behind a query are zeros, and zero times NaN or infinity would reach back in time: such
+      // values leave the product, and their columns are NaN from the first of them on.
+      if (poisoned) {
+        if (tid < COLS) {
+          int from = CHUNK;
+          for (int t = CHUNK - 1; t >= 0; --t) {
+            bf16 &v = s_v[t * LDV + tid];
+            if (!(fabsf(__bfloat162float(v)) < INFINITY)) from = t, v = __float2bfloat16_rn(0.0f);
+          }
+          s_bad[tid] = from;
+        }
+        __syncthreads();
       }
       if (mine) {
 #pragma unroll
@@ -525,6 +543,11 @@ decay_chunk_kernel(DecayArgs p) {
         if (t >= len || c >= cols) break;
         const float4 o4 = *reinterpret_cast<const float4 *>(s_o + t * LDO + c);
         float y[4] = {o4.x, o4.y, o4.z, o4.w};
+        if (poisoned) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (t >= s_bad[c + u]) y[u] = NAN;
+        }
         if constexpr (MEMORY) {
           const float den = s_den[t];
 #pragma unroll
