@@ -156,7 +156,7 @@ delta_chunk_numbers_kernel(DeltaArgs p) {
       dst[tid] = s_x[i][j] * s_beta[j];
       float px = 0.0f;
 #pragma unroll
-      for (int m = 0; m < CHUNK; ++m) px = fmaf(s_p[i][m], s_x[m][j], px);
+      for (int m = 0; m < CHUNK; ++m) px = m <= i ? fmaf(s_p[i][m], s_x[m][j], px) : px;
       dst[AT_P + tid] = px * s_beta[j];
       __syncthreads();                                  // s_g, s_beta, s_a, s_x and s_p are read
     }
@@ -268,20 +268,28 @@ delta_chunk_kernel(DeltaArgs p) {
       sq[0] += meet.part[w][CHUNK + i][c], sq[1] += meet.part[w + 1][CHUNK + i][c];
     }
     meet.rhs[i][c] = fmaf(-f[AT_GK + i], sk[0] + sk[1], __bfloat162float(s.v[i][c]));
-    float o = f[AT_GQ + i] * (sq[0] + sq[1]);
+    const float of_state = sq[0] + sq[1];
+    float o;
     __syncthreads();
     {
       float u[4] = {0.0f, 0.0f, 0.0f, 0.0f}, more[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
       for (int j = 0; j < CHUNK; j += 4) {
         const float4 m = *reinterpret_cast<const float4 *>(f + CHUNK * i + j), n = *reinterpret_cast<const float4 *>(f + AT_P + CHUNK * i + j);
-        const float r[4] = {meet.rhs[j][c], meet.rhs[j + 1][c], meet.rhs[j + 2][c], meet.rhs[j + 3][c]};
-        u[0] = fmaf(m.x, r[0], u[0]), u[1] = fmaf(m.y, r[1], u[1]), u[2] = fmaf(m.z, r[2], u[2]), u[3] = fmaf(m.w, r[3], u[3]);
-        more[0] = fmaf(n.x, r[0], more[0]), more[1] = fmaf(n.y, r[1], more[1]);
-        more[2] = fmaf(n.z, r[2], more[2]), more[3] = fmaf(n.w, r[3], more[3]);
+        // (both matrices are zero above the diagonal, or what a NaN made of it: later tokens stay out)
+        float r[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[e] = meet.rhs[j + e][c];
+        const float to_u[4] = {m.x, m.y, m.z, m.w}, to_o[4] = {n.x, n.y, n.z, n.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (j + e > i) continue;
+          u[e] = fmaf(to_u[e], r[e], u[e]);
+          more[e] = fmaf(to_o[e], r[e], more[e]);
+        }
       }
       meet.u[i][c] = (u[0] + u[1]) + (u[2] + u[3]);
-      o += (more[0] + more[1]) + (more[2] + more[3]);
+      o = fmaf(f[AT_GQ + i], of_state, (more[0] + more[1]) + (more[2] + more[3]));
     }
     if (chunk * CHUNK + i < q_len && e0 + c < p.vdim) dst[static_cast<int64_t>(chunk) * CHUNK * p.out_stride] = kept ? o : 0.0f;
     __syncthreads();

@@ -9,6 +9,7 @@ from test_gpu_recurrence_routes import DEV, cache_of, make_mixer, plain_products
 pytestmark = pytest.mark.gpu
 
 COLUMNS = {
+    "delta": {"q": (0, 256), "k": (256, 512), "v": (600, 601), "step": (1024, 1028), "decay": (1028, 1032)},
     "duality": {"x": (70, 71), "B": (256, 512), "C": (512, 768), "dt": (1024, 1028)},
     "memory": {"q": (0, 256), "k": (256, 512), "v": (700, 701), "i": (1536, 1538), "f": (1538, 1540)},
     "selective": {"x": (33, 34)},
