@@ -56,6 +56,15 @@ __device__ __forceinline__ void split_pair3(float x, float y, uint32_t &high, ui
   high = *reinterpret_cast<const uint32_t *>(&h);
   split_pair(x - low_of(high), y - high_of(high), mid, low);
 }
+// The same for a state, which may have overflown: an infinity is its first part, and the others are finite (inf - inf would
+// make the sum NaN; the minimum takes the bound, which lies above all rests).  What is within 2^-9 of the largest number
+// counts as overflown.
+__device__ __forceinline__ void split_state3(float x, float y, uint32_t &high, uint32_t &mid, uint32_t &low) {
+  constexpr float BOUND = 5.3e36f;         // 2^122
+  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+  high = *reinterpret_cast<const uint32_t *>(&h);
+  split_pair(fminf(x - low_of(high), BOUND), fminf(y - high_of(high), BOUND), mid, low);
+}
 __device__ __forceinline__ void copy16_async(void *dst, const void *src, bool live) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_addr(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
 }

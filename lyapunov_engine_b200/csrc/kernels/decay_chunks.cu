@@ -39,7 +39,7 @@
 namespace {
 
 using bf16 = __nv_bfloat16;
-using le::add4, le::high_of, le::ldsm4, le::ldsm4_trans, le::low_of, le::mma, le::mma_first, le::mma_split3, le::split_pair3;
+using le::add4, le::high_of, le::ldsm4, le::ldsm4_trans, le::low_of, le::mma, le::mma_first, le::mma_split3, le::split_pair3, le::split_state3;
 
 constexpr int CHUNK = 64;
 constexpr int SEGMENT = 256;
@@ -401,7 +401,7 @@ decay_chunk_kernel(DecayArgs p) {
           uint32_t a[3][4];
 #pragma unroll
           for (int u = 0; u < 4; ++u)
-            split_pair3(S[2 * ks + (u >> 1)][2 * (u & 1)], S[2 * ks + (u >> 1)][2 * (u & 1) + 1], a[0][u], a[1][u], a[2][u]);
+            split_state3(S[2 * ks + (u >> 1)][2 * (u & 1)], S[2 * ks + (u >> 1)][2 * (u & 1) + 1], a[0][u], a[1][u], a[2][u]);
 #pragma unroll
           for (int tb = 0; tb < CHUNK / 16; ++tb) {
             uint32_t qb[4];

@@ -38,7 +38,7 @@
 namespace {
 
 using bf16 = __nv_bfloat16;
-using le::ldsm4, le::ldsm4_trans, le::mma, le::mma_first, le::mma_split3, le::split_pair3;
+using le::ldsm4, le::ldsm4_trans, le::mma, le::mma_first, le::mma_split3, le::split_pair3, le::split_state3;
 
 constexpr int CHUNK = 16;
 constexpr int DIM = 128;                    // entries of a head, padded
@@ -244,7 +244,7 @@ delta_chunk_kernel(DeltaArgs p) {
     {
       uint32_t a[3][4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) split_pair3(S[u >> 1][2 * (u & 1)], S[u >> 1][2 * (u & 1) + 1], a[0][u], a[1][u], a[2][u]);
+      for (int u = 0; u < 4; ++u) split_state3(S[u >> 1][2 * (u & 1)], S[u >> 1][2 * (u & 1) + 1], a[0][u], a[1][u], a[2][u]);
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
         uint32_t vec[4];
