@@ -719,6 +719,7 @@ LE_API int le_duality_chunks(float *out, int64_t out_stride, const void *x, int6
   if (num_segments <= 0) return 0;
   if (heads < 1 || heads > 65535 || n_state < 1 || n_state > 128 || vdim < 1 || heads_per_group < 1 || num_segments > 65535)
     return le::invalid("le_duality_chunks: %d heads of %d x %d in %d segments", heads, vdim, n_state, num_segments);
+  if (!aligned(work, 16)) return le::invalid("le_duality_chunks: work has to start on 16 bytes");
   DecayArgs p = {};
   p.out = out, p.out_stride = out_stride;
   p.q = static_cast<const bf16 *>(bc) + c_col, p.k = static_cast<const bf16 *>(bc) + b_col, p.v = static_cast<const bf16 *>(x);
@@ -747,6 +748,7 @@ LE_API int le_memory_chunks(float *out, int64_t out_stride, const void *rows, in
   if (num_segments <= 0) return 0;
   if (heads < 1 || heads > 65535 || dim < 1 || dim > 128 || vdim < 1 || num_segments > 65535 || part_rows < 1 || vdim % part_rows)
     return le::invalid("le_memory_chunks: %d heads of %d x %d in %d segments", heads, dim, vdim, num_segments);
+  if (!aligned(work, 16)) return le::invalid("le_memory_chunks: work has to start on 16 bytes");
   if (!(cap > 0.0f)) return le::invalid("le_memory_chunks: the gates' cap must be positive");
   DecayArgs p = {};
   const bf16 *base = static_cast<const bf16 *>(rows);

@@ -1723,6 +1723,11 @@ def ssm_scan(out, x, bc, b_col: int, c_col: int, dt, z, dt_bias, a_log, d_skip, 
                               int(rows_per_group), 1 if per_row else 0, float(out_scale), _stream()), "le_ssm_scan")
 
 
+def _check_tiles(tile_request, tile_q0, count: int) -> None:
+    for t in (tile_request, tile_q0):
+        assert t.dtype == torch.int32 and t.is_contiguous() and t.numel() >= count
+
+
 _segment_sizes: dict[str, int] = {}
 SELECTIVE_MAX_STATE = 16           # numbers of state per row that the form over segments takes
 
@@ -1752,6 +1757,7 @@ def selective_segments(out, x, bc, b_col: int, c_col: int, dt, z, dt_bias, a_log
     assert n_state <= SELECTIVE_MAX_STATE and dt_bias.dtype == a_log.dtype == torch.float32 and a_log.is_contiguous()
     assert dt_bias.numel() == rows and a_log.numel() == rows * n_state
     assert d_skip is None or (d_skip.dtype == torch.float32 and d_skip.numel() == rows)
+    _check_tiles(tile_request, tile_q0, num_segments)
     assert scratch is None or (scratch.dtype == torch.float32 and scratch.is_contiguous()
                                and scratch.numel() >= num_segments * rows * (n_state + 1))
     _check(core().le_selective_segments(_ptr(out), dtype_code(out.dtype), out.stride(0), _ptr(x), x.stride(0), _ptr(bc),
@@ -1798,6 +1804,7 @@ def duality_chunks(out, x, bc, b_col: int, c_col: int, dt, z, dt_bias, a_log, d_
     assert n_state <= DECAY_CHUNK_MAX_DIM and rows_per_group % rows_per_head == 0
     assert dt_bias.dtype == a_log.dtype == torch.float32 and dt_bias.numel() == a_log.numel() == heads
     assert d_skip is None or (d_skip.dtype == torch.float32 and d_skip.numel() == heads)
+    _check_tiles(tile_request, tile_q0, num_segments)
     assert work.dtype == torch.float32 and work.is_contiguous() and work.numel() >= decay_work_floats(num_segments, T, heads, n_state)
     assert scratch is None or (scratch.dtype == torch.float32 and scratch.is_contiguous()
                                and scratch.numel() >= num_segments * rows * n_state)
@@ -1924,6 +1931,7 @@ def memory_chunks(out, rows, q_col: int, k_col: int, v_col: int, i_col: int, f_c
     _mlstm_checks(out, rows, i_bias, f_bias, state, heads, dim, vdim)
     T = rows.shape[0]
     assert rows.dtype == torch.bfloat16 and dim <= DECAY_CHUNK_MAX_DIM
+    _check_tiles(tile_request, tile_q0, num_segments)
     assert work.dtype == torch.float32 and work.is_contiguous() and work.numel() >= decay_work_floats(num_segments, T, heads, dim)
     assert scratch is None or (scratch.dtype == torch.float32 and scratch.is_contiguous()
                                and scratch.numel() >= num_segments * heads * (vdim + 1) * dim)
