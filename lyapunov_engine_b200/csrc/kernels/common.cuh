@@ -13,6 +13,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -50,6 +51,20 @@ inline int launched() {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) snprintf(error_buffer(), 512, "CUDA: %s", cudaGetErrorString(e));
   return static_cast<int>(e);
+}
+
+// Multiprocessors of the current device (148 where it cannot be asked), remembered per device.
+inline int multiprocessors() {
+  static std::atomic<int> known[64];
+  int device = 0, n = 0;
+  const bool asked = cudaGetDevice(&device) == cudaSuccess && device >= 0 && device < 64;
+  if (asked && (n = known[device].load(std::memory_order_relaxed)) > 0) return n;
+  if (asked && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && n > 0) {
+    known[device].store(n, std::memory_order_relaxed);
+    return n;
+  }
+  cudaGetLastError();
+  return 148;
 }
 
 // Programmatic dependent launch: a kernel launched with launch_chained() may

@@ -677,12 +677,8 @@ int launch_chunks(const DecayArgs &p, int segments, cudaStream_t stream) {
   constexpr size_t smem = decay_smem<DP, SUMS>();
   auto kernel = decay_chunk_kernel<DP, MEMORY, SUMS>;
   if (smem > 48 * 1024) {
-    static bool raised = false;                  // once per form and process
-    if (!raised) {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      if (e != cudaSuccess) return le::invalid("le_decay_chunks: cannot get %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-      raised = true;
-    }
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return le::invalid("le_decay_chunks: cannot get %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
   }
   const dim3 grid(p.heads * ((p.vdim + COLS - 1) / COLS), segments);
   return le::launch_chained(kernel, grid, dim3(THREADS), smem, stream, p);

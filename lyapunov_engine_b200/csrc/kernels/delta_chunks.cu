@@ -380,6 +380,6 @@ LE_API int le_gated_delta_chunks(float *out, int64_t out_stride, const void *qkv
   // Its blocks may come while the kernel before it still holds multiprocessors, and would then share the others while
   // those stay idle (blocks of the form with four tokens, four to a multiprocessor: 1,040 us instead of 380).  Where every
   // block can have a multiprocessor of its own it asks for more than half of the shared memory, so that each gets one.
-  if (static_cast<int64_t>(grid.x) * grid.y * grid.z <= 148) return launch_walk<8>(p, grid, 116 * 1024, stream);
+  if (static_cast<int64_t>(grid.x) * grid.y * grid.z <= le::multiprocessors()) return launch_walk<8>(p, grid, 116 * 1024, stream);
   return launch_walk<4>(p, grid, 0, stream);
 }

@@ -220,15 +220,8 @@ constexpr F32Shape F32_SHAPES[] = {
     {48, 64, 33.0f, 42.0f, launch_f32<8, 6, 4, 16, 4>},   {64, 128, 48.0f, 100.0f, launch_f32<8, 8, 8, 32, 3>},
 };
 
-int multiprocessors() {
-  int device = 0, sms = 0;
-  if (cudaGetDevice(&device) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0) return sms;
-  cudaGetLastError();
-  return 148;
-}
-
 const F32Shape *best_shape(int M, int N) {
-  static const int sms = multiprocessors();
+  const int sms = le::multiprocessors();
   const F32Shape *best = nullptr;
   float least = 0.0f;
   for (const F32Shape &s : F32_SHAPES) {
