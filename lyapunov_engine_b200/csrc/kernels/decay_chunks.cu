@@ -103,15 +103,18 @@ __device__ __forceinline__ double chunk_sum(double x, double *totals) {
   __syncthreads();
   return (warp & 1) ? x + totals[warp - 1] : x;
 }
+// e^L for a sum in 64 bits: both of its floats count.
+__device__ __forceinline__ float exp_of_sum(float high, float low) {
+  const float e = le::exp_unbiased(high);
+  return fmaf(e, low, e);                                  // (low is no more than a rounding of high)
+}
+__device__ __forceinline__ float exp_of_sum(double L) {
+  const float high = static_cast<float>(L);
+  return exp_of_sum(high, static_cast<float>(L - static_cast<double>(high)));
+}
 __device__ __forceinline__ float4 gate_of(double L, float w, float floor) {
   const float high = static_cast<float>(L);
   return make_float4(high, static_cast<float>(L - static_cast<double>(high)), w, floor);
-}
-
-// e^(high + low), low no more than a rounding of high.
-__device__ __forceinline__ float exp_of_sum(float high, float low) {
-  const float e = le::exp_unbiased(high);
-  return fmaf(e, low, e);
 }
 
 // State-space duality: one block per segment and head, a thread per token.
@@ -136,7 +139,7 @@ duality_gates_kernel(DecayArgs p, const bf16 *dt_rows, int64_t dt_stride, const 
     double all = 0.0;
 #pragma unroll
     for (int w = 0; w < SEGMENT / 32; ++w) all += totals[w];
-    p.keeps[static_cast<int64_t>(seg) * p.heads + head] = le::exp_unbiased(static_cast<float>(all));
+    p.keeps[static_cast<int64_t>(seg) * p.heads + head] = exp_of_sum(all);
   }
 }
 
@@ -195,7 +198,7 @@ memory_gates_kernel(DecayArgs p, const bf16 *rows, int64_t row_stride, int i_col
       double all = 0.0;
 #pragma unroll
       for (int w = 0; w < SEGMENT / 32; ++w) all += totals[w];
-      p.keeps[static_cast<int64_t>(at) * p.heads + head] = le::exp_unbiased(static_cast<float>(all));
+      p.keeps[static_cast<int64_t>(at) * p.heads + head] = exp_of_sum(all);
     }
     ++at;
     run = s_run;

@@ -184,3 +184,24 @@ def test_requests_without_a_state_row_leave_everything_alone():
                           torch.zeros(H, device=DEV), state, i32([-1]), i32([0, T]), i32([0, 0]), i32([0, 256]), 2, H, d, e, 5.0, 0.25,
                           work, scratch)
     assert float(out.abs().max()) == 0.0 and bool((state == 4.0).all())
+
+
+def test_a_segments_decay_keeps_all_bits_of_its_sum():
+    """Keys of zeros: the state behind the request is its first state times all decays, from one segment to the next."""
+    from lyapunov_engine_b200 import ops
+    H, P, N, T = 64, 8, 8, 3 * 256
+    R = H * P
+    rows = torch.zeros(T, R + 2 * N + H, device=DEV, dtype=torch.bfloat16)
+    rows[:, R + 2 * N:] = torch.randn(T, H, generator=torch.Generator(device=DEV).manual_seed(4), device=DEV).bfloat16()
+    zeros, a_log = torch.zeros(H, device=DEV), torch.linspace(-5.0, -3.0, H, device=DEV)    # sums of -2 to -14 a segment
+    state = torch.ones(1, R, N, device=DEV)
+    out, n = torch.empty(T, R, device=DEV), T // ops.decay_segment()
+    ops.duality_chunks(out, rows[:, :R], rows, R, R + N, rows[:, R + 2 * N:], None, zeros, a_log, zeros, state, i32([0]), i32([0, T]),
+                       i32([0] * n), i32(range(0, T, 256)), n, N, P, R, torch.empty(ops.decay_work_floats(n, T, H, N), device=DEV),
+                       torch.empty(n, R, N, device=DEV))
+    # three segments' exponentials, a unit in the last place of each at most (2^-23), and two products (2^-24 each); what the
+    # 768 logarithms' own roundings differ by, to both sides, is a hundredth of that
+    dt = torch.nn.functional.softplus(rows[:, R + 2 * N:].float())
+    logs = (-dt * torch.exp(a_log)).double().sum(0)
+    off = (state.view(H, -1).double() / torch.exp(logs)[:, None] - 1.0).abs()
+    assert float(off.max()) <= 8 * 2.0 ** -24, float(off.max())
