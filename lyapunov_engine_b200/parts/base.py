@@ -188,6 +188,11 @@ class PositionEncoding(Part):
 WHOLE = 1 << 30
 
 
+def portions(ctx) -> tuple[int, int]:
+    """(tokens of a step's longest request, requests with several tokens): what the recurrent mixers choose a form by."""
+    return ctx.max_q_len, ctx.num_requests - ctx.num_decode
+
+
 class Mixer(Part):
     # a bias [H] (32-bit) on the output that forward() leaves to the block that adds the output to the stream (named
     # by ``o_bias_name``; blocks that add none refuse such a mixer)

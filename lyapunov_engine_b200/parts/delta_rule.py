@@ -17,8 +17,8 @@ matrix per request and head (``state_need``); the convolutions' last taps - 1
 inputs are state of the request too (``extra_state_needs``).  One product makes
 all six projections; the convolution, the recurrence and the gated norm are a
 kernel each (ops.short_conv_general, ops.gated_delta_scan, ops.head_norm_gate);
-requests that bring several tokens in bfloat16, heads of 65 to 128 entries, go
-over chunks on the tensor cores (ops.gated_delta_chunks).
+requests that bring more than a few tokens in bfloat16, heads of 65 to 128
+entries, go over chunks on the tensor cores (ops.gated_delta_chunks).
 Unit vectors, decays, step sizes, the recurrence and the norm are 32-bit.
 """
 from __future__ import annotations
@@ -26,9 +26,16 @@ from __future__ import annotations
 import torch
 
 from .. import ops
-from .base import WHOLE, Mixer, StateNeed, TensorDecl, register_mixer
+from .base import WHOLE, Mixer, StateNeed, TensorDecl, portions, register_mixer
 
 UNIT_EPS = 1e-6
+
+
+def over_chunks(longest: int, requests: int) -> bool:
+    """Whether portions are long enough for the chunked form: a chunk of 16 costs the same however few of its tokens there
+    are, the scan goes token by token (16 heads of 128 x 128, us, scan against chunks: one request of 8 tokens 7 / 9, of 24
+    13 / 10, of 32 17 / 11; 2 of 24 14 / 15; 3 of 24 14 / 17, of 32 18 / 17; 6 of 16 19 / 17; 8 of 8 17 / 20; 32 of 4 43 / 48)."""
+    return longest >= 32 or (longest >= 16 and longest * requests >= 96)
 
 
 @register_mixer("gated_delta")
@@ -117,13 +124,14 @@ class GatedDeltaMixer(Mixer):
                 cache.state, ctx.state_slots, ctx.cu_q)
         sizes = (H, G, d, e, UNIT_EPS, d ** -0.5)
         request, _, _, several = ctx.tiles[WHOLE]
-        if several and self.chunks:
+        over = several > 0 and self.chunks and over_chunks(*portions(ctx))
+        if over:
             numbers = ws.get("delta_chunks", (ops.gated_delta_chunk_floats(T, ctx.num_requests, H),), torch.float32)
             ops.gated_delta_chunks(*rows, request, several, *sizes, numbers)
         # decoded tokens keep the scan, whatever stands beside them in the step
-        if not (several and self.chunks) or ctx.num_decode:
+        if not over or ctx.num_decode:
             scratch = ws.get("delta_numbers", (T, ops.gated_delta_scratch_width(H, G)), torch.float32)
-            if several and self.chunks:
+            if over:
                 ops.gated_delta_scan(*rows, ctx.num_decode, *sizes, scratch=scratch, requests=ctx.decode_requests)
             else:
                 ops.gated_delta_scan(*rows, ctx.num_requests, *sizes, scratch=scratch)

@@ -13,18 +13,24 @@ With x the mixer's input, H heads, d the query/key size and e the value size:
 S, n and m are carried from token to token in 32 bits, per request and head
 (``state_need``).  One product makes all six projections; the recurrence and
 the gated norm are a kernel each (ops.mlstm_scan, ops.head_norm_gate); requests
-that bring several tokens in bfloat16 go over chunks on the tensor cores
-(ops.memory_chunks).  The
-gates, the recurrence and the norm are 32-bit.
+that bring more than a few tokens in bfloat16 go over chunks on the tensor
+cores (ops.memory_chunks).  The gates, the recurrence and the norm are 32-bit.
 """
 from __future__ import annotations
 
 import torch
 
 from .. import ops
-from .base import Mixer, StateNeed, TensorDecl, register_mixer
+from .base import Mixer, StateNeed, TensorDecl, portions, register_mixer
 
 SEGMENT = 256      # tokens of a request that a block of the chunked form takes
+
+
+def over_chunks(longest: int, requests: int) -> bool:
+    """Whether portions are long enough for the chunked form.  Two launches and a chunk of 64 cost the same however few
+    tokens there are; the scan goes token by token (8 heads of 128 x 256, us, scan against chunks: one request of 24 tokens
+    15 / 16, of 32 18 / 16; 8 of 12 22 / 25, of 16 28 / 25; 16 of 8 32 / 39, of 12 42 / 39; 32 of 4 42 / 59)."""
+    return longest >= 28 or (longest >= 12 and longest * requests >= 112)
 
 
 @register_mixer("matrix_memory")
@@ -101,7 +107,7 @@ class MatrixMemoryMixer(Mixer):
                 ctx.state_slots, ctx.cu_q)
         sizes = (H, d, e, self.gate_cap, d ** -0.5)
         request, q0, _, segments = ctx.tiles[SEGMENT]
-        if segments and rt.dtype == torch.bfloat16 and d <= ops.DECAY_CHUNK_MAX_DIM:
+        if segments and rt.dtype == torch.bfloat16 and d <= ops.DECAY_CHUNK_MAX_DIM and over_chunks(*portions(ctx)):
             # (a step in which no request has a second segment goes from state row to state row)
             scratch = None
             if segments > ctx.num_requests - ctx.num_decode:

@@ -20,10 +20,11 @@ G)), inner = H * P:
     y <- y * silu(z);  W_o
 
 Both recurrences run in one kernel (ops.ssm_scan), with the gate in its
-epilogue; requests that bring several tokens in bfloat16 go through the duality
-over chunks on the tensor cores (ops.duality_chunks) and through the selective
-scan over segments side by side (ops.selective_segments) instead.  The
-convolution is the package's short convolution with a bias and silu; the last taps - 1 inputs of the convolution are state of the request too
+epilogue; requests that bring more than a few tokens in bfloat16 go through the
+duality over chunks on the tensor cores (ops.duality_chunks) and through the
+selective scan over segments side by side (ops.selective_segments) instead.  The
+convolution is the package's short convolution with a bias and silu; the last
+taps - 1 inputs of the convolution are state of the request too
 (``extra_state_needs``).  Step sizes, decays, the recurrence and the norm are
 32-bit.
 """
@@ -32,10 +33,29 @@ from __future__ import annotations
 import torch
 
 from .. import ops
-from .base import Mixer, StateNeed, TensorDecl, register_mixer
+from .base import Mixer, StateNeed, TensorDecl, portions, register_mixer
 
 SELECTIVE_SEGMENT = 64   # tokens of a request that a block of the selective scan's form over segments takes
 SEGMENT = 256      # tokens of a request that a block of the duality's chunked form takes
+
+
+def duality_over_chunks(longest: int, requests: int) -> bool:
+    """Whether portions are long enough for the duality over chunks.  Two launches and a chunk of 64 cost the same however
+    few tokens there are; the scan goes token by token (64 heads of 64 x 128, us, scan against chunks: one request of 16
+    tokens 12 / 14, of 32 22 / 16; 2 of 24 20 / 22; 6 of 8 21 / 21, of 12 27 / 21; 8 of 8 26 / 29; 32 of 4 73 / 90, of 8
+    99 / 92)."""
+    return longest >= 28 or (longest >= 8 and longest * requests >= 72)
+
+
+def scan_over_segments(longest: int, requests: int) -> bool:
+    """Whether portions are long enough for the selective scan over segments.  Within one segment a thread walks a row's
+    whole state where the scan spreads it over lanes: better only where there are rows enough.  Beyond, three launches, two
+    of which walk 64 tokens, against one that walks all (2,048 channels of 16, us, scan against segments: 1 of 64 22 / 34,
+    2 of 32 17 / 18, 3 of 32 21 / 18; 1 of 128 43 / 77, of 256 84 / 88; 2 of 128 69 / 90, of 224 124 / 87; 3 of 192 117 / 120;
+    8 of 96 85 / 93, of 128 113 / 101; 16 of 65 115 / 116)."""
+    if longest <= SELECTIVE_SEGMENT:
+        return requests >= 3
+    return longest * (requests + 3) >= 1152
 
 
 def _conv(out, rows, channels, mixer, ctx, cache):
@@ -144,7 +164,7 @@ class StateSpaceDualityMixer(Mixer):
                 proj[:, self.z_col:self.z_col + inner], self.dt_bias, self.a_log, self.d_skip, cache.state, ctx.state_slots, ctx.cu_q)
         sizes = (N, self.value_dim, (H // self.groups) * self.value_dim)
         request, q0, _, segments = ctx.tiles[SEGMENT]
-        if segments and rt.dtype == torch.bfloat16 and N <= ops.DECAY_CHUNK_MAX_DIM:
+        if segments and rt.dtype == torch.bfloat16 and N <= ops.DECAY_CHUNK_MAX_DIM and duality_over_chunks(*portions(ctx)):
             # (a step in which no request has a second segment goes from state row to state row)
             scratch = None
             if segments > ctx.num_requests - ctx.num_decode:
@@ -248,7 +268,7 @@ class SelectiveScanMixer(Mixer):
         rows = (out, conv, low, self.b_col, self.c_col, dt, proj[:, self.z_col:self.z_col + C], self.dt_bias, self.a_log,
                 self.d_skip, cache.state, ctx.state_slots, ctx.cu_q)
         request, q0, _, segments = ctx.tiles[SELECTIVE_SEGMENT]
-        if segments and rt.dtype == torch.bfloat16 and N <= ops.SELECTIVE_MAX_STATE:
+        if segments and rt.dtype == torch.bfloat16 and N <= ops.SELECTIVE_MAX_STATE and scan_over_segments(*portions(ctx)):
             # (a step in which no request has a second segment goes from state row to state row)
             scratch = None
             if segments > ctx.num_requests - ctx.num_decode:

@@ -53,7 +53,10 @@ def cache_of(mixer, rows, seed=3):
     g = torch.Generator(device=DEV).manual_seed(seed)
     def fresh(need):
         return torch.randn((rows, *need.shape), generator=g, device=DEV) * 0.2
-    return SimpleNamespace(state=fresh(mixer.state_need()), extra={k: fresh(v) for k, v in mixer.extra_state_needs().items()})
+    state = fresh(mixer.state_need())
+    if hasattr(mixer, "gate_cap"):
+        state.zero_()                                   # (the memory's parts hold copies of one vector)
+    return SimpleNamespace(state=state, extra={k: fresh(v) for k, v in mixer.extra_state_needs().items()})
 
 
 @pytest.fixture
@@ -84,3 +87,39 @@ def test_a_decoded_tokens_bits_do_not_depend_on_prompts_beside_it(kind, plain_pr
     assert bool((mixed.state[0] != alone.state[0]).any())
     for slot in (1, 3, 5):
         assert torch.equal(mixed.state[slot], alone.state[slot])
+
+
+FORMS = {"delta": ("gated_delta_chunks", "gated_delta_scan"), "duality": ("duality_chunks", "ssm_scan"),
+         "selective": ("selective_segments", "ssm_scan"), "memory": ("memory_chunks", "mlstm_scan")}
+
+
+@pytest.mark.parametrize("kind,q_lens,over", [
+    ("delta", [15], False), ("delta", [32], True), ("delta", [16, 1, 1], False), ("delta", [16] * 6, True),
+    ("duality", [8], False), ("duality", [28, 1], True), ("duality", [7] * 32, False), ("duality", [9] * 8, True),
+    ("selective", [64], False), ("selective", [200], False), ("selective", [288], True), ("selective", [5] * 3, True),
+    ("selective", [80] * 8, False), ("selective", [65] * 16, True),
+    ("memory", [27], False), ("memory", [28], True), ("memory", [8] * 20, False), ("memory", [14] * 8, True)])
+def test_short_portions_stay_with_the_scan(kind, q_lens, over, plain_products, monkeypatch):
+    """Both sides of each rule; results of the two routes agree."""
+    from lyapunov_engine_b200 import ops
+    m, called = make_mixer(kind), []
+    for name in FORMS[kind]:
+        def entry(*args, _name=name, _entry=getattr(ops, name), **kwargs):
+            called.append(_name)
+            return _entry(*args, **kwargs)
+        monkeypatch.setattr(ops, name, entry)
+    x = torch.randn(sum(q_lens), 16, generator=torch.Generator(device=DEV).manual_seed(1), device=DEV).bfloat16()
+    step = step_of(m, q_lens, list(range(len(q_lens))))
+    cache = cache_of(m, len(q_lens))
+    got = m.forward(x, step, cache)
+    assert set(called) == ({FORMS[kind][0]} | ({FORMS[kind][1]} if 1 in q_lens else set()) if over else {FORMS[kind][1]})
+    # token by token
+    plain, t0 = cache_of(m, len(q_lens)), 0
+    for b, n in enumerate(q_lens):
+        want = torch.cat([m.forward(x[t:t + 1], step_of(m, [1], [b]), plain).clone() for t in range(t0, t0 + n)])
+        # (the norm's rounding to bfloat16 on top of 32-bit sums in another order)
+        torch.testing.assert_close(got[t0:t0 + n].float(), want.float(), atol=1e-3, rtol=2.0 ** -7)
+        t0 += n
+        if b == 2:
+            break
+    torch.testing.assert_close(cache.state[:min(3, len(q_lens))], plain.state[:min(3, len(q_lens))], atol=3e-5, rtol=3e-5)
