@@ -507,10 +507,17 @@ sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int v
     float best = -INFINITY;
     int idx = 0x7fffffff;
     bool odd = false;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const float x = vals[i];
-      if (x != x) odd = true;
-      if (x > best || (x == best && begin + i < idx)) { best = x; idx = begin + i; }
+    if (filtered) {
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const float x = vals[i];
+        if (x != x) odd = true;
+        if (x > best || (x == best && begin + i < idx)) { best = x; idx = begin + i; }
+      }
+    } else {
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const float x = vals[i];
+        if (x > best || (x == best && begin + i < idx)) { best = x; idx = begin + i; }
+      }
     }
     // for a row with filters: the smallest of the threads' maxima (a thread without a value stands aside; NaN: -inf)
     if (filtered) {
