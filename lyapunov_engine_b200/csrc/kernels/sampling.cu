@@ -126,7 +126,7 @@ __global__ void argmax_final_kernel(int32_t *__restrict__ out, const float *__re
 //
 // The two thresholds need no sort.  First by value: bins of equal width below the row's maximum (linear_select), which
 // a row's values fall into evenly, so that plain atomic additions do; the few values of the bin that a threshold lies in
-// are then compared with one another.  Where that cannot be done (a bin with too many values, rows with NaN or infinite
+// are then compared with one another.  Where that cannot be done (too many values close together, rows with NaN or infinite
 // maxima, more values to keep than there are threads) by radix selection over the ordered bit patterns, 11 + 11 + 10 bits.  A level
 // makes a histogram (count, and for top-p the probability mass, per digit) of the row's values whose higher
 // digits are the ones chosen so far; block 0 adds the blocks' histograms up and picks the digit the threshold
@@ -160,6 +160,7 @@ struct SampleShared {
   unsigned long long above;                // what lies above the bin the threshold falls into, and that bin
   int bin;
   int listed[2];                           // block 0: values of that bin
+  uint32_t least, most;                    // block 0: the smallest and the largest of their keys, where they are too many
   uint32_t chosen[2];                      // block 0: the threshold
   // what every block tells the others
   float block_max;
@@ -334,7 +335,11 @@ __device__ uint32_t radix_select(cg::cluster_group &cluster, SampleShared &h, Me
 // limit the smallest.  `limit`: top_p of all mass, or k - 1.  The first levels of the radix selection put a row's values
 // into some 40 bins (sign, exponent, two bits): a warp's lanes had to be sorted out by bin before they could add, twelve
 // groups one after the other, which was the time of a row with top_p (one row of 128,256: 92 us, of which a row without
-// filters takes 17; now 27).  False: the radix selection has to do it.
+// filters takes 17; now 27).
+// A bin with more values than the list takes (a row whose values lie close together beside its temperature): they are all
+// the same, or a second level makes bins of their ordered bit patterns, which are even enough within one bin of the first.
+// (With the radix selection behind a list too long, such rows paid for both: one of 128,256 at temperature 2.5 109 us, a
+// flat one 71, where the radix selection alone takes 97 and 43.)  False: the radix selection has to do it.
 constexpr int LIST_MAX = 512;              // (every value of the list meets every other)
 struct BinList {
   unsigned long long mass[LIST_MAX];
@@ -342,26 +347,28 @@ struct BinList {
 };
 static_assert(sizeof(BinList) <= sizeof(MergedHistogram), "the list lies where the merged histogram does");
 
-__device__ bool linear_select(cg::cluster_group &cluster, SampleShared &h, BinList *list, int which, const float *vals, int n,
-                              bool with_mass, int k, float top_p, uint32_t min_key, float row_max, float inv_t, float scale,
-                              uint32_t &threshold) {
+// One level: a histogram of the values that take part, its sums over the cluster, the bin in which the sum from `base` on
+// passes the limit (what lies above it: `above`), and that bin's values in block 0's list.  bin_of(x, key): a value's bin,
+// or -1: it takes no part; limit_of(total): the limit.  False: the sum does not pass it.
+template <typename BinOf, typename MassOf, typename LimitOf>
+__device__ __forceinline__ bool select_level(cg::cluster_group &cluster, SampleShared &h, BinList *list, int which, const float *vals,
+                                             int n, unsigned long long base, BinOf bin_of, MassOf mass_of, LimitOf limit_of,
+                                             int &bin, unsigned long long &above, unsigned long long &limit) {
   constexpr int SHARE = RADIX_BINS / SAMPLE_BLOCKS;
   const int rank = static_cast<int>(cluster.block_rank()), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  auto bin_of = [&](float x) { return static_cast<int>(fminf((row_max - x) * scale, static_cast<float>(RADIX_BINS - 1))); };
-  auto mass_of = [&](float x) -> unsigned long long { return with_mass ? __float2ull_rd(prob_of(x, row_max, inv_t) * MASS_ONE) : 1ull; };
-  for (int bin = threadIdx.x; bin < RADIX_BINS; bin += blockDim.x) h.mass_lo[bin] = 0, h.mass_hi[bin] = 0;
+  for (int b = threadIdx.x; b < RADIX_BINS; b += blockDim.x) h.mass_lo[b] = 0, h.mass_hi[b] = 0;
   if (threadIdx.x == 0) h.listed[which] = 0, h.chosen[which] = 0xffffffffu;
   __syncthreads();
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const float x = vals[i];
-    if (ordered_key(x) < min_key) continue;
+    const int at = bin_of(x, ordered_key(x));
+    if (at < 0) continue;
     const unsigned long long m = mass_of(x);
     if (m == 0) continue;
-    const int bin = bin_of(x);
     const unsigned add_lo = static_cast<unsigned>(m), add_hi = static_cast<unsigned>(m >> 32);
-    const unsigned old = atomicAdd(&h.mass_lo[bin], add_lo);
+    const unsigned old = atomicAdd(&h.mass_lo[at], add_lo);
     const unsigned carry = old + add_lo < old ? 1u : 0u;              // additions with carry commute: the sum is exact
-    if (add_hi + carry) atomicAdd(&h.mass_hi[bin], add_hi + carry);
+    if (add_hi + carry) atomicAdd(&h.mass_hi[at], add_hi + carry);
   }
   cluster.sync();                          // every block's histogram is there
   // this block's share of the bins, summed over the blocks and scanned: warps 0 .. SHARE / 32 - 1, a bin a lane
@@ -387,51 +394,113 @@ __device__ bool linear_select(cg::cluster_group &cluster, SampleShared &h, BinLi
     if (threadIdx.x == SHARE - 1) h.share[which] = upto;
   }
   cluster.sync();                          // every block's share is summed
-  unsigned long long total = 0, before = 0;
+  unsigned long long total = 0, before = base;
   for (int other = 0; other < SAMPLE_BLOCKS; ++other) {
-    if (other == rank) before = total;
+    if (other == rank) before = base + total;
     total += cluster.map_shared_rank(&h, other)->share[which];
   }
-  const unsigned long long limit = with_mass ? __double2ull_rd(static_cast<double>(top_p) * static_cast<double>(total))
-                                             : static_cast<unsigned long long>(k - 1);
-  if (total <= limit) return false;        // (every block sees the same)
+  limit = limit_of(total);
+  if (base + total <= limit) return false; // (every block sees the same)
   if (threadIdx.x < SHARE && before + upto - mine <= limit && before + upto > limit) h.bin = my_bin, h.above = before + upto - mine;
   int owner = -1;                          // the last block up to whose share the sum stays within the limit
-  for (unsigned long long sum = 0; owner + 1 < SAMPLE_BLOCKS && sum <= limit;) sum += cluster.map_shared_rank(&h, ++owner)->share[which];
+  for (unsigned long long sum = base; owner + 1 < SAMPLE_BLOCKS && sum <= limit;) sum += cluster.map_shared_rank(&h, ++owner)->share[which];
   cluster.sync();                          // the owner of that bin has found it
   const SampleShared *from = cluster.map_shared_rank(&h, owner);
-  const int bin = from->bin;
-  const unsigned long long above = from->above;
+  bin = from->bin;
+  above = from->above;
   SampleShared *first = cluster.map_shared_rank(&h, 0);
   BinList *all = cluster.map_shared_rank(list, 0);
   const int rounds = (n + blockDim.x - 1) / blockDim.x;
   for (int round = 0; round < rounds; ++round) {
     const int i = round * blockDim.x + threadIdx.x;
     const float x = i < n ? vals[i] : 0.0f;
-    bool in = i < n && ordered_key(x) >= min_key && bin_of(x) == bin;
+    bool in = i < n && bin_of(x, ordered_key(x)) == bin;
     unsigned long long m = 0;
     if (in) m = mass_of(x), in = m != 0;   // (a value without mass is no threshold)
     const unsigned found = __ballot_sync(0xffffffffu, in);
     if (found == 0) continue;
     int at = 0;
     if (lane == 0) at = atomicAdd(&first->listed[which], __popc(found));
-    at = __shfl_sync(0xffffffffu, at, 0) + __popc(found & ((1u << lane) - 1u));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (at >= LIST_MAX) break;             // (too many already)
+    at += __popc(found & ((1u << lane) - 1u));
     if (in && at < LIST_MAX) all->key[at] = ordered_key(x), all->mass[at] = m;
   }
   cluster.sync();                          // the list is complete
-  const int listed = first->listed[which];
-  if (listed > LIST_MAX) {
-    cluster.sync();                        // (nobody clears the list's place while another still reads its length)
-    return false;
-  }
-  if (rank == 0 && threadIdx.x < listed) {
+  return true;
+}
+
+// The threshold from a list that holds all values of its bin.
+__device__ __forceinline__ uint32_t from_list(cg::cluster_group &cluster, SampleShared &h, const BinList *list, int which, int listed,
+                                              unsigned long long above, unsigned long long limit, uint32_t min_key) {
+  if (cluster.block_rank() == 0 && threadIdx.x < listed) {
     const uint32_t key = list->key[threadIdx.x];
     unsigned long long sum = above;
     for (int i = 0; i < listed; ++i) sum += list->key[i] > key ? list->mass[i] : 0ull;
     if (sum <= limit) atomicMin(&h.chosen[which], key);
   }
   cluster.sync();
-  threshold = max(first->chosen[which], min_key);
+  return max(cluster.map_shared_rank(&h, 0)->chosen[which], min_key);
+}
+
+// Behind a first level whose list was too short for `bin`.
+__device__ __noinline__ bool refine_select(SampleShared &h, BinList *list, int which, const float *vals, int n, bool with_mass,
+                                           uint32_t min_key, float row_max, float inv_t, float scale, int bin,
+                                           unsigned long long above, unsigned long long limit, uint32_t &threshold) {
+  cg::cluster_group cluster = cg::this_cluster();
+  SampleShared *first = cluster.map_shared_rank(&h, 0);
+  auto mass_of = [&](float x) -> unsigned long long { return with_mass ? __float2ull_rd(prob_of(x, row_max, inv_t) * MASS_ONE) : 1ull; };
+  // the smallest and the largest of the bin's keys
+  if (threadIdx.x == 0) h.least = 0xffffffffu, h.most = 0;
+  cluster.sync();                          // (and everyone has read the list's length)
+  uint32_t lo = 0xffffffffu, hi = 0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const float x = vals[i];
+    const uint32_t key = ordered_key(x);
+    if (key < min_key || static_cast<int>(fminf((row_max - x) * scale, static_cast<float>(RADIX_BINS - 1))) != bin || mass_of(x) == 0) continue;
+    lo = min(lo, key), hi = max(hi, key);
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo), hi = __reduce_max_sync(0xffffffffu, hi);
+  if ((threadIdx.x & 31) == 0 && lo <= hi) {
+    atomicMin(&first->least, lo);
+    atomicMax(&first->most, hi);
+  }
+  cluster.sync();
+  lo = first->least, hi = first->most;
+  if (lo == hi) {
+    threshold = lo;
+    return true;
+  }
+  const int shift = max(0, 21 - __clz(static_cast<int>(hi - lo)));    // (hi - lo) >> shift is below 2,048
+  auto bin_of = [&](float, uint32_t key) { return key >= lo && key <= hi ? static_cast<int>((hi - key) >> shift) : -1; };
+  const unsigned long long base = above;
+  if (!select_level(cluster, h, list, which, vals, n, base, bin_of, mass_of, [&](unsigned long long) { return limit; }, bin, above, limit))
+    return false;
+  const int listed = first->listed[which];
+  if (listed > LIST_MAX) {
+    cluster.sync();                        // (nobody clears the list's place while another still reads its length)
+    return false;
+  }
+  threshold = from_list(cluster, h, list, which, listed, above, limit, min_key);
+  return true;
+}
+
+__device__ bool linear_select(cg::cluster_group &cluster, SampleShared &h, BinList *list, int which, const float *vals, int n,
+                              bool with_mass, int k, float top_p, uint32_t min_key, float row_max, float inv_t, float scale,
+                              uint32_t &threshold) {
+  auto bin_of = [&](float x, uint32_t key) {
+    return key < min_key ? -1 : static_cast<int>(fminf((row_max - x) * scale, static_cast<float>(RADIX_BINS - 1)));
+  };
+  auto mass_of = [&](float x) -> unsigned long long { return with_mass ? __float2ull_rd(prob_of(x, row_max, inv_t) * MASS_ONE) : 1ull; };
+  auto limit_of = [&](unsigned long long total) {
+    return with_mass ? __double2ull_rd(static_cast<double>(top_p) * static_cast<double>(total)) : static_cast<unsigned long long>(k - 1);
+  };
+  int bin = 0;
+  unsigned long long above = 0, limit = 0;
+  if (!select_level(cluster, h, list, which, vals, n, 0ull, bin_of, mass_of, limit_of, bin, above, limit)) return false;
+  const int listed = cluster.map_shared_rank(&h, 0)->listed[which];
+  if (listed > LIST_MAX) return refine_select(h, list, which, vals, n, with_mass, min_key, row_max, inv_t, scale, bin, above, limit, threshold);
+  threshold = from_list(cluster, h, list, which, listed, above, limit, min_key);
   return true;
 }
 
@@ -595,7 +664,8 @@ sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int v
     // have one.
     const float scale = static_cast<float>(RADIX_BINS - 1) / (row_max - row_floor);
     const int threads = min(vocab, (vocab / slice) * static_cast<int>(blockDim.x));
-    if (!(plain && k <= threads && scale > 0.0f && scale < INFINITY &&
+    if (plain && k <= threads && row_floor == row_max && row_max != 0.0f) keep_key = ordered_key(row_max);   // k maxima (0: of two signs)
+    else if (!(plain && k <= threads && scale > 0.0f && scale < INFINITY &&
           linear_select(cluster, sh, list, 0, vals, n, false, k, 1.0f, 0u, row_max, inv_t, scale, keep_key)))
       keep_key = radix(false, k, 1.0f, 0u);
   }

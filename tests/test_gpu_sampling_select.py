@@ -21,6 +21,10 @@ def rows_of(kind, n, vocab, g):
         gone = torch.rand(n, vocab, generator=g, device=DEV) < 0.7
         gone[:, vocab // 2] = False              # (a row without any value has no distribution)
         return x.masked_fill(gone, -float("inf"))
+    if kind == "close":                          # many values to a bin: a second level of bins
+        return x * 0.02
+    if kind == "ulps":                           # neighbouring numbers, each many times
+        return 1.0 + torch.randint(0, 3000, x.shape, generator=g, device=DEV) * 2.0 ** -23
     if kind == "two":
         return (x > 0).float()
     if kind == "one":
@@ -29,7 +33,7 @@ def rows_of(kind, n, vocab, g):
     return x
 
 
-@pytest.mark.parametrize("kind", ["normal", "rounded", "flat", "masked", "two", "one"])
+@pytest.mark.parametrize("kind", ["normal", "rounded", "flat", "masked", "two", "one", "close", "ulps"])
 @pytest.mark.parametrize("vocab,n", [(5, 13), (1023, 13), (8200, 26), (32768, 13), (128256, 26), (300000, 13)])
 def test_kept_sets(vocab, n, kind):
     from lyapunov_engine_b200 import ops
