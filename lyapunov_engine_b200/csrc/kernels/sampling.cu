@@ -533,7 +533,7 @@ __device__ float block_inclusive_scan(float v, float *warp_f, float &block_total
 // TO_A_SM: blocks a multiprocessor is to hold.  Two (32 registers a thread, some 40 spilled) where there are more blocks
 // than multiprocessors: the waits of one block's meetings are the other's time (64 rows of 128,256 with all kinds of options:
 // 234 us before the selection by value, 107 with it, 96 with two blocks).  One otherwise (a row with top_p 27 us, with
-// 32 registers 31).
+// 32 registers 31); blocks_to_a_multiprocessor() draws the line.
 // slice: values per block (a multiple of 4); `staged`: the slice fits in shared memory and is copied there.
 template <int TO_A_SM>
 __global__ void __launch_bounds__(THREADS, TO_A_SM)
@@ -776,6 +776,70 @@ LE_API int le_argmax(int32_t *out, const float *logits, int num_rows, int vocab,
                             static_cast<const int32_t *>(part_idx), chunks);
 }
 
+namespace {
+
+constexpr size_t MAX_SLICE_BYTES = 152 * 1024;
+
+// A block's share of a row, whether it is copied into shared memory (where it fits beside the histograms: vocabularies up
+// to about 300,000), and the shared memory that takes.
+size_t slice_smem(int vocab, int &slice, int &staged) {
+  slice = ((vocab + SAMPLE_BLOCKS - 1) / SAMPLE_BLOCKS + 3) / 4 * 4;
+  const size_t slice_bytes = static_cast<size_t>(slice) * sizeof(float);
+  staged = slice_bytes <= MAX_SLICE_BYTES ? 1 : 0;
+  return sizeof(MergedHistogram) + (staged ? slice_bytes : 0);
+}
+
+// (the same for every vocabulary: another thread's call must not lower it again)
+cudaError_t raise_sample_smem() {
+  constexpr int most = static_cast<int>(sizeof(MergedHistogram) + MAX_SLICE_BYTES);
+  cudaError_t e = cudaFuncSetAttribute(sample_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(sample_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
+// Which form a launch takes, asked of the device once per size of shared memory: one block to a multiprocessor where all
+// rows' clusters run at once that way (clusters stay inside one part of the chip: some 16 rows, not 148 / 8), two where two
+// fit (vocabularies up to about 131,000).  128,256 words, rows with top-k, us, one block against two: 16 rows 49 / 43
+// (two waves against one); 151,936 words, where one block fits: 64 rows 140 with 64 registers a thread, 151 with the 32 of
+// the form for two.
+int blocks_to_a_multiprocessor(int num_rows, size_t smem) {
+  struct Known {
+    int device = -1;
+    size_t smem = 0;
+    int rows = 0;                          // that run at once, one block to a multiprocessor
+    bool two = false;
+  };
+  thread_local Known known;
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) device = 0;
+  if (known.device != device || known.smem != smem) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(SAMPLE_BLOCKS, 1);
+    config.blockDim = dim3(THREADS);
+    config.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = SAMPLE_BLOCKS;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    config.attrs = attr;
+    config.numAttrs = 1;
+    int rows = 0, blocks = 0;
+    if (cudaOccupancyMaxActiveClusters(&rows, sample_kernel<1>, &config) != cudaSuccess) rows = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, sample_kernel<2>, THREADS, smem) != cudaSuccess) blocks = 0;
+    cudaGetLastError();                    // a refusal is an answer, not an error of the caller
+    known.device = device, known.smem = smem, known.rows = rows, known.two = blocks >= 2;
+  }
+  return num_rows > known.rows && known.two ? 2 : 1;
+}
+
+}  // namespace
+
+// The form that le_sample takes: blocks to a multiprocessor.
+LE_API int le_sample_blocks(int num_rows, int vocab) {
+  int slice = 0, staged = 0;
+  const size_t smem = slice_smem(vocab, slice, staged);
+  return raise_sample_smem() == cudaSuccess ? blocks_to_a_multiprocessor(num_rows, smem) : 0;
+}
+
 // seeds: [rows, 3] = seed low word, seed high word, counter.  `uniforms`
 // (optional) overrides the generator; `probs_out` (optional, [rows, vocab])
 // receives the filtered distribution, for tests.
@@ -784,17 +848,11 @@ LE_API int le_sample(int32_t *out, const float *logits, int num_rows, int vocab,
                      const float *uniforms, float *probs_out, cudaStream_t stream) {
   if (num_rows <= 0) return 0;
   if (num_rows > 65535) return le::invalid("le_sample: too many rows for one launch");
-  int slice = (vocab + SAMPLE_BLOCKS - 1) / SAMPLE_BLOCKS;
-  slice = (slice + 3) / 4 * 4;
-  // the slice is copied into shared memory where it fits beside the histograms (vocabularies up to about 300,000)
-  const size_t slice_bytes = static_cast<size_t>(slice) * sizeof(float);
-  const int staged = slice_bytes <= 152 * 1024 ? 1 : 0;
-  const size_t smem = sizeof(MergedHistogram) + (staged ? slice_bytes : 0);
-  auto *kernel = num_rows * SAMPLE_BLOCKS > 148 ? sample_kernel<2> : sample_kernel<1>;
-  {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return le::invalid("le_sample: cannot get %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-  }
+  int slice = 0, staged = 0;
+  const size_t smem = slice_smem(vocab, slice, staged);
+  if (cudaError_t e = raise_sample_smem(); e != cudaSuccess)
+    return le::invalid("le_sample: cannot get %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+  auto *kernel = blocks_to_a_multiprocessor(num_rows, smem) == 2 ? sample_kernel<2> : sample_kernel<1>;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(SAMPLE_BLOCKS, num_rows);
   config.blockDim = dim3(THREADS);

@@ -63,3 +63,14 @@ def test_kept_sets(vocab, n, kind):
             assert float(mass[stays & (x[i] >= least)].sum()) >= (top_p - 2e-5) * float(all_mass)
         else:
             assert bool((kept == seen).all())
+
+
+def test_two_blocks_to_a_multiprocessor_only_where_two_fit():
+    """The form with half the registers: where one block a multiprocessor means a second wave, and two blocks fit."""
+    from lyapunov_engine_b200 import ops
+    form = ops.core().le_sample_blocks
+    for vocab in (1000, 32000, 128256):
+        forms = [form(n, vocab) for n in (1, 8, 16, 17, 19, 32, 64)]
+        assert forms[:2] == [1, 1] and forms[-2:] == [2, 2] and forms == sorted(forms)
+    for vocab in (151936, 256000, 300000):
+        assert [form(n, vocab) for n in (1, 19, 64)] == [1, 1, 1]
