@@ -583,6 +583,7 @@ sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int v
         if (x > best || (x == best && begin + i < idx)) { best = x; idx = begin + i; }
       }
     } else {
+#pragma unroll 4
       for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const float x = vals[i];
         if (x > best || (x == best && begin + i < idx)) { best = x; idx = begin + i; }
