@@ -2,6 +2,8 @@
 type, scratch memory and the device status word."""
 from __future__ import annotations
 
+import math
+
 import torch
 
 from .. import ops
@@ -40,6 +42,23 @@ class Workspace:
         if type(shape) is tuple and len(self._views) < 4096:
             self._views[(name, shape, dtype)] = view
         return view
+
+    def parts(self, name: str, shapes: tuple, dtype) -> tuple:
+        """Several buffers of one type as one, each on 16 bytes: what a part
+        needs beside a large buffer does not cost an allocation of its own."""
+        views = self._views.get((name, shapes, dtype))
+        if views is not None:
+            return views
+        starts, n = [], 0
+        step = 16 // dtype.itemsize
+        for shape in shapes:
+            starts.append(n)
+            n += (math.prod(shape) + step - 1) // step * step
+        whole = self.get(name, (n,), dtype)
+        views = tuple(whole[a:a + math.prod(shape)].view(*shape) for a, shape in zip(starts, shapes))
+        if len(self._views) < 4096:
+            self._views[(name, shapes, dtype)] = views
+        return views
 
     def bytes(self) -> int:
         return sum(b.numel() * b.element_size() for b in self._buffers.values())

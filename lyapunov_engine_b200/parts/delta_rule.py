@@ -119,22 +119,24 @@ class GatedDeltaMixer(Mixer):
             tile_request, tile_q0, num_tiles, _ = ctx.tiles[ops.SHORT_CONV_TILE]
             ops.short_conv_general(conv, proj[:, :self.channels], self.w_taps, taps_state, ctx.state_slots, ctx.cu_q,
                                    tile_request, tile_q0, num_tiles, add_input=False, silu=True)
-        o = ws.get("delta_out", (T, H * e), torch.float32)
+        request, _, _, several = ctx.tiles[WHOLE]
+        over = several > 0 and self.chunks and over_chunks(*portions(ctx))
+        scans = not over or ctx.num_decode > 0      # decoded tokens keep the scan, whatever stands beside them in the step
+        shapes = ((T, H * e),)
+        if over:
+            shapes += ((ops.gated_delta_chunk_floats(T, ctx.num_requests, H),),)
+        if scans:
+            shapes += ((T, ops.gated_delta_scratch_width(H, G)),)
+        o, *scratch = ws.parts("delta_out", shapes, torch.float32)
         rows = (o, conv, self.q_col, self.k_col, self.v_col, proj, self.beta_col, self.decay_col, self.a_log, self.dt_bias,
                 cache.state, ctx.state_slots, ctx.cu_q)
         sizes = (H, G, d, e, UNIT_EPS, d ** -0.5)
-        request, _, _, several = ctx.tiles[WHOLE]
-        over = several > 0 and self.chunks and over_chunks(*portions(ctx))
         if over:
-            numbers = ws.get("delta_chunks", (ops.gated_delta_chunk_floats(T, ctx.num_requests, H),), torch.float32)
-            ops.gated_delta_chunks(*rows, request, several, *sizes, numbers)
-        # decoded tokens keep the scan, whatever stands beside them in the step
-        if not over or ctx.num_decode:
-            scratch = ws.get("delta_numbers", (T, ops.gated_delta_scratch_width(H, G)), torch.float32)
-            if over:
-                ops.gated_delta_scan(*rows, ctx.num_decode, *sizes, scratch=scratch, requests=ctx.decode_requests)
-            else:
-                ops.gated_delta_scan(*rows, ctx.num_requests, *sizes, scratch=scratch)
+            ops.gated_delta_chunks(*rows, request, several, *sizes, scratch[0])
+        if scans and over:
+            ops.gated_delta_scan(*rows, ctx.num_decode, *sizes, scratch=scratch[-1], requests=ctx.decode_requests)
+        elif scans:
+            ops.gated_delta_scan(*rows, ctx.num_requests, *sizes, scratch=scratch[-1])
         gated = ws.get("delta_gated", (T, H * e), rt.dtype)
         ops.head_norm_gate(gated, o, proj[:, self.gate_col:self.gate_col + H * e], self.norm_weight, self.norm_eps, H, e)
         return ops.linear_for_residual(gated, self.w_o, ws, "mixer_out", ctx.status)

@@ -102,18 +102,20 @@ class MatrixMemoryMixer(Mixer):
         T = x.shape[0]
         proj = ws.get("mlstm_proj", (T, self.width), rt.dtype)
         ops.linear(proj, x, self.w_in, ctx.status)
-        o = ws.get("mlstm_out", (T, H * e), torch.float32)
+        request, q0, _, segments = ctx.tiles[SEGMENT]
+        over = segments > 0 and rt.dtype == torch.bfloat16 and d <= ops.DECAY_CHUNK_MAX_DIM and over_chunks(*portions(ctx))
+        shapes = ((T, H * e),)
+        if over:
+            # (a step in which no request has a second segment goes from state row to state row, without scratch)
+            shapes += ((ops.decay_work_floats(segments, T, H, d),),)
+            if segments > ctx.num_requests - ctx.num_decode:
+                shapes += ((segments, H, e + 1, d),)
+        o, *work = ws.parts("mlstm_out", shapes, torch.float32)
         rows = (o, proj, self.q_col, self.k_col, self.v_col, self.i_col, self.f_col, self.i_bias, self.f_bias, cache.state,
                 ctx.state_slots, ctx.cu_q)
         sizes = (H, d, e, self.gate_cap, d ** -0.5)
-        request, q0, _, segments = ctx.tiles[SEGMENT]
-        if segments and rt.dtype == torch.bfloat16 and d <= ops.DECAY_CHUNK_MAX_DIM and over_chunks(*portions(ctx)):
-            # (a step in which no request has a second segment goes from state row to state row)
-            scratch = None
-            if segments > ctx.num_requests - ctx.num_decode:
-                scratch = ws.get("mlstm_scratch", (segments, H, e + 1, d), torch.float32)
-            work = ws.get("mlstm_work", (ops.decay_work_floats(segments, T, H, d),), torch.float32)
-            ops.memory_chunks(*rows, request, q0, segments, *sizes, work, scratch)
+        if over:
+            ops.memory_chunks(*rows, request, q0, segments, *sizes, work[0], work[1] if len(work) > 1 else None)
             if ctx.num_decode:
                 ops.mlstm_scan(*rows, ctx.num_decode, *sizes, requests=ctx.decode_requests)
         else:

@@ -159,18 +159,20 @@ class StateSpaceDualityMixer(Mixer):
         ops.linear(proj, x, self.w_in, ctx.status)
         conv = ws.get("ssd_conv", (T, self.channels), rt.dtype)
         _conv(conv, proj, self.channels, self, ctx, cache)
-        y = ws.get("ssd_y", (T, inner), torch.float32)
+        request, q0, _, segments = ctx.tiles[SEGMENT]
+        over = segments > 0 and rt.dtype == torch.bfloat16 and N <= ops.DECAY_CHUNK_MAX_DIM and duality_over_chunks(*portions(ctx))
+        shapes = ((T, inner),)
+        if over:
+            # (a step in which no request has a second segment goes from state row to state row, without scratch)
+            shapes += ((ops.decay_work_floats(segments, T, H, N),),)
+            if segments > ctx.num_requests - ctx.num_decode:
+                shapes += ((segments, inner, N),)
+        y, *work = ws.parts("ssd_y", shapes, torch.float32)
         rows = (y, conv[:, :inner], conv, inner, inner + self.groups * N, proj[:, self.dt_col:self.dt_col + H],
                 proj[:, self.z_col:self.z_col + inner], self.dt_bias, self.a_log, self.d_skip, cache.state, ctx.state_slots, ctx.cu_q)
         sizes = (N, self.value_dim, (H // self.groups) * self.value_dim)
-        request, q0, _, segments = ctx.tiles[SEGMENT]
-        if segments and rt.dtype == torch.bfloat16 and N <= ops.DECAY_CHUNK_MAX_DIM and duality_over_chunks(*portions(ctx)):
-            # (a step in which no request has a second segment goes from state row to state row)
-            scratch = None
-            if segments > ctx.num_requests - ctx.num_decode:
-                scratch = ws.get("ssd_scratch", (segments, inner, N), torch.float32)
-            work = ws.get("ssd_work", (ops.decay_work_floats(segments, T, H, N),), torch.float32)
-            ops.duality_chunks(*rows, request, q0, segments, *sizes, work, scratch)
+        if over:
+            ops.duality_chunks(*rows, request, q0, segments, *sizes, work[0], work[1] if len(work) > 1 else None)
             if ctx.num_decode:
                 ops.ssm_scan(*rows, ctx.num_decode, *sizes, per_row=False, requests=ctx.decode_requests)
         else:
