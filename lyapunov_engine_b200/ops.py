@@ -1736,6 +1736,8 @@ SELECTIVE_MAX_STATE = 16           # numbers of state per row that the form over
 def selective_segment() -> int:
     """Tokens per segment of selective_segments()."""
     if "selective" not in _segment_sizes:
+        if core().le_selective_max_state() != SELECTIVE_MAX_STATE:
+            raise KernelError(f"the kernels' segments take {core().le_selective_max_state()} numbers of state, not {SELECTIVE_MAX_STATE}")
         _segment_sizes["selective"] = int(core().le_selective_segment())
     return _segment_sizes["selective"]
 

@@ -171,18 +171,24 @@ def test_matrix_memory_over_chunks(shape, cut):
         assert float((off / size).max()) <= 4e-6 + 8 * cap * 2.0 ** -23
 
 
-def test_requests_without_a_state_row_leave_everything_alone():
+@pytest.mark.parametrize("T", [300, 100])                        # (two segments with scratch, one without)
+def test_requests_without_a_state_row_leave_everything_alone(T):
     """Slot -1 (padding of a fixed-shape step): zeros out, no state touched."""
     from lyapunov_engine_b200 import ops
-    H, d, e, T = 2, 16, 24, 300
+    H, d, e = 2, 16, 24
+    n = (T + 255) // 256
+    lists = (i32([-1]), i32([0, T]), i32([0] * n), i32(256 * s for s in range(n)), n)
     rows = torch.randn(T, 2 * H * d + H * e + 16, device=DEV).bfloat16()
-    state = torch.full((3, *ops.mlstm_state_shape(H, d, e)), 4.0, device=DEV)
-    out = torch.full((T, H * e), 9.0, device=DEV)
-    work = torch.empty(ops.decay_work_floats(2, T, H, d), device=DEV)
-    for scratch in (torch.empty(2, H, e + 1, d, device=DEV),):
-        ops.memory_chunks(out, rows, 0, H * d, 2 * H * d, 2 * H * d + H * e, 2 * H * d + H * e + H, torch.zeros(H, device=DEV),
-                          torch.zeros(H, device=DEV), state, i32([-1]), i32([0, T]), i32([0, 0]), i32([0, 256]), 2, H, d, e, 5.0, 0.25,
-                          work, scratch)
+    zeros, work = torch.zeros(H, device=DEV), torch.empty(ops.decay_work_floats(n, T, H, d), device=DEV)
+
+    state, out = torch.full((3, *ops.mlstm_state_shape(H, d, e)), 4.0, device=DEV), torch.full((T, H * e), 9.0, device=DEV)
+    ops.memory_chunks(out, rows, 0, H * d, 2 * H * d, 2 * H * d + H * e, 2 * H * d + H * e + H, zeros, zeros, state, *lists, H, d, e,
+                      5.0, 0.25, work, torch.empty(n, H, e + 1, d, device=DEV) if n > 1 else None)
+    assert float(out.abs().max()) == 0.0 and bool((state == 4.0).all())
+
+    state, out = torch.full((3, H * e, d), 4.0, device=DEV), torch.full((T, H * e), 9.0, device=DEV)
+    ops.duality_chunks(out, rows[:, 2 * H * d:2 * H * d + H * e], rows, 0, d, rows[:, 2 * H * d + H * e:], None, zeros, zeros, zeros, state,
+                       *lists, d, e, H * e, work, torch.empty(n, H * e, d, device=DEV) if n > 1 else None)
     assert float(out.abs().max()) == 0.0 and bool((state == 4.0).all())
 
 
