@@ -29,9 +29,10 @@
 //
 // What bounds it, and the layout that follows: token by token (one request, 64 heads of 64 x 128,
 // 2,048 tokens) a prompt is 2,048 steps of load, multiply-add, shuffle, each as long as their latencies
-// (1,310 us; the matrix memory of 8 heads of 128 x 256 1,090 us).  A chunk is one step instead, and segments of
-// SEGMENT tokens run side by side: every segment's own sum first (SUMS), then the states they start from, element
-// by element, then the outputs.  A block is one segment, one head and 64 columns of S; S^T stays in the
+// (1,268 us, over chunks 165; the matrix memory of 8 heads of 128 x 256 1,019 us, 126).  A chunk is one step
+// instead, and segments of SEGMENT tokens run side by side: every segment's own sum first (SUMS), then the states
+// they start from, element by element, then the outputs (35, 11 and 135 us cold; the tensor pipes are busy for a
+// third and a fifth of them).  A block is one segment, one head and 64 columns of S; S^T stays in the
 // accumulators of its four warps (16 columns each, all of dim), whose layout is that of the left operand of the
 // next product, so the state never passes through shared memory.
 #include "chunk_mma.cuh"
@@ -48,7 +49,7 @@ constexpr int THREADS = 128;
 constexpr int LDV = COLS + 8;       // rows of v, of the weighted scores (bfloat16) and of outputs (float) in shared
 constexpr int LDP = CHUNK + 8;      // memory: padded so that eight rows' 16-byte pieces fall into different banks
 constexpr int LDO = COLS + 4;
-constexpr float SMALLEST_LOG = -1.0e4f;   // of one token's decay: its exponential is zero by far, and sums stay finite
+constexpr float SMALLEST_LOG = -1.0e4f;   // of one token's decay: its exponential is exp_unbiased's smallest, 1.6e-38, and sums stay finite
 
 __device__ __forceinline__ float softplus_f32(float v) { return v > 20.0f ? v : log1pf(expf(v)); }
 __device__ __forceinline__ float log_sigmoid_f32(float x) {
@@ -227,8 +228,9 @@ decay_chunk_kernel(DecayArgs p) {
   float *s_o = reinterpret_cast<float *>(s_p);             // [CHUNK][LDO]: outputs, once the scores are used
   float *s_hi = reinterpret_cast<float *>(s_p + (SUMS ? 0 : 3 * CHUNK * LDP)), *s_lo = s_hi + CHUNK, *s_w = s_lo + CHUNK;
   float *s_from = s_w + CHUNK, *s_to = s_from + CHUNK;     // e^(L_i), e^(L_last - L_j) w_j
-  // Of a pair of tokens in different sixteens the weight is a product: from the key to the end of its sixteen, from there
-  // to the start of the query's, from there to the query; none of the three is above 1, and none is an exponential per pair.
+  // Of a pair of tokens in different sixteens the weight is a product: from the key to the end of its sixteen (times the
+  // key's w), from there to the start of the query's, from there to the query; none of the three decays is above 1, and
+  // none is an exponential per pair.
   float *s_in = s_to + CHUNK, *s_out = s_in + CHUNK, *s_over = s_out + CHUNK;      // s_over [4][4]
   float *s_floor = s_over + 16, *s_row = s_floor + CHUNK, *s_den = s_row + CHUNK;
   float *s_n = s_den + CHUNK;                              // [DP]

@@ -27,12 +27,12 @@
 // the two small products with the right sides are 32-bit multiply-adds; the update multiplies
 // u in three parts with exact k.  All sums are 32-bit.
 //
-// What bounds it: token by token (3,001 tokens, 16 heads of 128 x 128) a prompt was
+// What bounds it: token by token (3,001 tokens, 16 heads of 128 x 128) a prompt is
 // 3,001 steps of dots, shuffles and updates, each as long as its latencies, behind
-// warps that fetched one batch after the other (563 us; four tokens at a time in
-// 32-bit multiply-adds 437 us).  A chunk is four meetings of the block instead:
-// 232 us, of which the numbers take 30 (u and o one after the other 248).  Error
-// against 64 bits 2.25e-6, before 2.30e-6.
+// warps that fetch one batch after the other (539 us; four tokens at a time in
+// 32-bit multiply-adds it was 437).  A chunk is four meetings of the block instead:
+// 227 us, of which the numbers take 30 (u and o one after the other 248).  Error
+// against 64 bits over 1,024 tokens 2.7e-7 to 6.0e-7, the scan's 2.8e-7 to 6.6e-7.
 #include "chunk_mma.cuh"
 
 namespace {

@@ -247,7 +247,7 @@ ssm_scan_kernel(SsmArgs p) {
 // ---------------------------------------------------------------- segments of tokens side by side
 // The form with a decay per row and state for requests that bring several tokens (bfloat16 rows, one group, up to
 // SEG_STATE numbers of state per row).  Walked token by token a prompt is a chain of dependent steps and a request's
-// rows are all the threads there are (2,048 rows of 16 numbers, 2,048 tokens: 601 us, now 164 us; error against 64 bits
+// rows are all the threads there are (2,048 rows of 16 numbers, 2,048 tokens: 664 us, over segments 160; error against 64 bits
 // 1.62e-7, now 1.47e-7).  Here segments of SEG_TOKENS tokens run side by side, a thread per row with the row's whole
 // state in registers:
 //   selective_segment_kernel<SUMS>   each segment from a zero state: the state it ends in, and the sum of its step sizes
