@@ -1411,6 +1411,42 @@ def graph_median_us(launch, sets):
     return times[len(times) // 2]
 
 
+def segments_of(tokens, size, dev):
+    """The tile lists of one request of ``tokens`` tokens in segments of ``size``, and their number."""
+    import torch
+
+    n = (tokens + size - 1) // size
+    return (torch.zeros(n, dtype=torch.int32, device=dev), torch.arange(0, n * size, size, dtype=torch.int32, device=dev), n)
+
+
+def memory_launch(rows, states, slots, cu, reqs, tokens, heads, dim, vdim, dev):
+    """The matrix memory as a step runs it: decoded tokens through the scan, a prompt over chunks."""
+    import torch
+
+    from lyapunov_engine_b200 import ops
+
+    if tokens <= 64:
+        return lambda i: ops.mlstm_scan(*rows, states[i], slots, cu, reqs, heads, dim, vdim, 15.0, dim ** -0.5)
+    tr, tq, n = segments_of(tokens, ops.decay_segment(), dev)
+    work = torch.empty(ops.decay_work_floats(n, tokens, heads, dim), device=dev)
+    parts = torch.empty(n, heads, vdim + 1, dim, device=dev)
+    return lambda i: ops.memory_chunks(*rows, states[i], slots, cu, tr, tq, n, heads, dim, vdim, 15.0, dim ** -0.5, work, parts)
+
+
+def delta_launch(rows, states, slots, cu, reqs, tokens, heads, kv_heads, dim, vdim, dev):
+    """The gated delta rule as a step runs it: decoded tokens through the scan, a prompt over chunks."""
+    import torch
+
+    from lyapunov_engine_b200 import ops
+
+    if tokens <= 64:
+        return lambda i: ops.gated_delta_scan(*rows, states[i], slots, cu, reqs, heads, kv_heads, dim, vdim, 1e-6, dim ** -0.5)
+    listed = torch.arange(reqs, dtype=torch.int32, device=dev)
+    numbers = torch.empty(ops.gated_delta_chunk_floats(tokens, reqs, heads), device=dev)
+    return lambda i: ops.gated_delta_chunks(*rows, states[i], slots, cu, listed, reqs, heads, kv_heads, dim, vdim, 1e-6, dim ** -0.5,
+                                            numbers)
+
+
 def zepilix_kernel_rows(pk, llama):
     """Each kernel the design adds, alone, beside the like kernel of the closest existing path at the same sizes:
     microseconds per launch inside a captured graph over rotating tensors, the share of the measured copy bandwidth
@@ -1497,9 +1533,10 @@ def zepilix_kernel_rows(pk, llama):
         o = torch.empty(T, H * e, device=dev)
         a_log, dt_bias = torch.zeros(H, device=dev), torch.zeros(H, device=dev)
         conv.normal_()
-        row(f"delta rule, {H} heads of {d} x {e}, {reqs} request(s)", "", T, reqs * 2 * 4 * H * d * e + T * (C * 2 + H * e * 4),
-            lambda i: ops.gated_delta_scan(o, conv, 0, G * d, 2 * G * d, proj, C + H * e, C + H * e + H, a_log, dt_bias, states[i],
-                                           slots, cu, reqs, H, G, d, e, 1e-6, d ** -0.5), state_sets, fp32_flops=6 * T * H * d * e)
+        row(f"delta rule{'' if T <= 64 else ' over chunks'}, {H} heads of {d} x {e}, {reqs} request(s)", "", T,
+            reqs * 2 * 4 * H * d * e + T * (C * 2 + H * e * 4),
+            delta_launch((o, conv, 0, G * d, 2 * G * d, proj, C + H * e, C + H * e + H, a_log, dt_bias), states, slots, cu, reqs, T, H, G, d,
+                         e, dev), state_sets, fp32_flops=6 * T * H * d * e)
         gated = torch.empty(T, H * e, device=dev, dtype=bf)
         wn = torch.ones(e, device=dev)
         row("norm per head times silu gate", "", T, T * H * e * 8, lambda i: ops.head_norm_gate(gated, o, proj[:, C:C + H * e], wn, 1e-6, H, e), 1)
@@ -1722,6 +1759,7 @@ def ribozen_kernel_rows(pk, llama):
     dm, mm, pm = cfg["layers"][0]["mixer"], cfg["layers"][2]["mixer"], cfg["layers"][3]["mixer"]
     for T in (8, 2048):
         reqs = T if T <= 64 else 1
+        over = "" if T <= 64 else " over chunks"      # as a step runs them: decoded tokens through the scans, prompts over chunks
         q_lens = [T // reqs] * reqs
         cu = torch.tensor([0] + list(torch.tensor(q_lens).cumsum(0)), dtype=torch.int32, device=dev)
         slots = torch.arange(reqs, dtype=torch.int32, device=dev)
@@ -1734,10 +1772,17 @@ def ribozen_kernel_rows(pk, llama):
         y = torch.empty(T, inner, device=dev)
         states = [torch.zeros(reqs + 1, inner, N, device=dev) for _ in range(state_sets)]
         zeros_h = torch.zeros(H, device=dev)
-        row(f"state-space recurrence, {H} heads of {P} x {N} (one decay per head), {reqs} request(s)",
-            "delta rule, 16 heads of 128 x 128", T, reqs * 2 * 4 * inner * N + T * (C * 2 + inner * 6 + H * 2),
-            lambda i: ops.ssm_scan(y, conv[:, :inner], conv, inner, inner + G * N, proj[:, inner:inner + H], proj[:, :inner], zeros_h,
-                                   zeros_h, zeros_h, states[i], slots, cu, reqs, N, P, (H // G) * P, per_row=False), state_sets,
+        args = lambda i: (y, conv[:, :inner], conv, inner, inner + G * N, proj[:, inner:inner + H], proj[:, :inner], zeros_h, zeros_h,
+                          zeros_h, states[i], slots, cu)
+        if T <= 64:
+            launch = lambda i: ops.ssm_scan(*args(i), reqs, N, P, (H // G) * P, per_row=False)
+        else:
+            tr, tq, n = segments_of(T, ops.decay_segment(), dev)
+            work = torch.empty(ops.decay_work_floats(n, T, H, N), device=dev)
+            parts = torch.empty(n, inner, N, device=dev)
+            launch = lambda i: ops.duality_chunks(*args(i), tr, tq, n, N, P, (H // G) * P, work, parts)
+        row(f"state-space recurrence{over}, {H} heads of {P} x {N} (one decay per head), {reqs} request(s)",
+            "delta rule, 16 heads of 128 x 128", T, reqs * 2 * 4 * inner * N + T * (C * 2 + inner * 6 + H * 2), launch, state_sets,
             fp32_flops=6 * T * inner * N)
         normed = torch.empty(T, inner, device=dev, dtype=bf)
         wn = torch.ones(inner, device=dev)
@@ -1754,10 +1799,16 @@ def ribozen_kernel_rows(pk, llama):
         outs = torch.empty(T, Cs, device=dev, dtype=bf)
         states = [torch.zeros(reqs + 1, Cs, Ns, device=dev) for _ in range(state_sets)]
         a_log, zeros_c = torch.zeros(Cs, Ns, device=dev), torch.zeros(Cs, device=dev)
-        row(f"state-space recurrence, {Cs} channels x {Ns} (a decay per channel and state), {reqs} request(s)",
-            "delta rule, 16 heads of 128 x 128", T, reqs * 2 * 4 * Cs * Ns + 4 * Cs * Ns + T * (Cs * 8 + Ns * 4),
-            lambda i: ops.ssm_scan(outs, convs, low, R, R + Ns, dt, z, zeros_c, a_log, zeros_c, states[i], slots, cu, reqs, Ns, 1, Cs,
-                                   per_row=True, out_scale=1.0), state_sets, fp32_flops=6 * T * Cs * Ns)
+        args = lambda i: (outs, convs, low, R, R + Ns, dt, z, zeros_c, a_log, zeros_c, states[i], slots, cu)
+        if T <= 64:
+            launch = lambda i: ops.ssm_scan(*args(i), reqs, Ns, 1, Cs, per_row=True)
+        else:
+            tr, tq, n = segments_of(T, ops.selective_segment(), dev)
+            parts = torch.empty(n, Cs, Ns + 1, device=dev)
+            launch = lambda i: ops.selective_segments(*args(i), tr, tq, n, Ns, parts)
+        row(f"state-space recurrence{over.replace('chunks', 'segments')}, {Cs} channels x {Ns} (a decay per channel and state), "
+            f"{reqs} request(s)", "delta rule, 16 heads of 128 x 128", T, reqs * 2 * 4 * Cs * Ns + 4 * Cs * Ns + T * (Cs * 8 + Ns * 4),
+            launch, state_sets, fp32_flops=6 * T * Cs * Ns)
         del states
         # matrix memory
         Hm, d, e = mm["heads"], mm["dim"], mm["vdim"]
@@ -1766,11 +1817,10 @@ def ribozen_kernel_rows(pk, llama):
         o = torch.empty(T, Hm * e, device=dev)
         states = [torch.zeros(reqs + 1, *ops.mlstm_state_shape(Hm, d, e), device=dev) for _ in range(state_sets)]
         zeros_m = torch.zeros(Hm, device=dev)
-        row(f"matrix memory, {Hm} heads of {d} x {e}, {reqs} request(s)", "delta rule, 16 heads of 128 x 128", T,
+        row(f"matrix memory{over}, {Hm} heads of {d} x {e}, {reqs} request(s)", "delta rule, 16 heads of 128 x 128", T,
             reqs * 2 * states[0][0].numel() * 4 + T * (width * 2 + Hm * e * 4),
-            lambda i: ops.mlstm_scan(o, rows_m, 0, Hm * d, 2 * Hm * d, 2 * Hm * d + 2 * Hm * e, 2 * Hm * d + 2 * Hm * e + Hm, zeros_m,
-                                     zeros_m, states[i], slots, cu, reqs, Hm, d, e, 15.0, d ** -0.5), state_sets,
-            fp32_flops=4 * T * Hm * d * (e + 1))
+            memory_launch((o, rows_m, 0, Hm * d, 2 * Hm * d, 2 * Hm * d + 2 * Hm * e, 2 * Hm * d + 2 * Hm * e + Hm, zeros_m, zeros_m),
+                          states, slots, cu, reqs, T, Hm, d, e, dev), state_sets, fp32_flops=4 * T * Hm * d * (e + 1))
         gated = torch.empty(T, Hm * e, device=dev, dtype=bf)
         wm = torch.ones(Hm * e, device=dev)
         row("norm per head (a weight per head) times sigmoid gate", "norm per head times silu gate", T, T * Hm * e * 8,
@@ -1785,10 +1835,9 @@ def ribozen_kernel_rows(pk, llama):
         od = torch.empty(T, Hd * dd, device=dev)
         states = [torch.zeros(reqs + 1, Hd, dd, dd, device=dev) for _ in range(state_sets)]
         zeros_d = torch.zeros(Hd, device=dev)
-        row(f"delta rule, {Hd} heads of {dd} x {dd}, {reqs} request(s)", "", T, reqs * 2 * 4 * Hd * dd * dd + T * (Cd * 2 + Hd * dd * 4),
-            lambda i: ops.gated_delta_scan(od, convd, 0, Gd * dd, 2 * Gd * dd, projd, Cd + Hd * dd, Cd + Hd * dd + Hd, zeros_d, zeros_d,
-                                           states[i], slots, cu, reqs, Hd, Gd, dd, dd, 1e-6, dd ** -0.5), state_sets,
-            fp32_flops=6 * T * Hd * dd * dd)
+        row(f"delta rule{over}, {Hd} heads of {dd} x {dd}, {reqs} request(s)", "", T, reqs * 2 * 4 * Hd * dd * dd + T * (Cd * 2 + Hd * dd * 4),
+            delta_launch((od, convd, 0, Gd * dd, 2 * Gd * dd, projd, Cd + Hd * dd, Cd + Hd * dd + Hd, zeros_d, zeros_d), states, slots, cu,
+                         reqs, T, Hd, Gd, dd, dd, dev), state_sets, fp32_flops=6 * T * Hd * dd * dd)
         del states
         # bias, norm over whole projections, turn, cache write; beside the turn of pairs with its norm per head
         pages = (T + page - 1) // page + 1
@@ -2045,9 +2094,10 @@ def zuzenex_kernel_rows(pk, llama):
         om = torch.empty(T, Hm * em, device=dev)
         states = [torch.zeros(reqs + 1, *ops.mlstm_state_shape(Hm, 128, em), device=dev) for _ in range(sets)]
         zeros_m = torch.zeros(Hm, device=dev)
-        row(f"matrix memory, {Hm} heads of 128 x {em}, {reqs} request(s)", "", T, reqs * 2 * states[0][0].numel() * 4 + T * (wm * 2 + Hm * em * 4),
-            lambda i: ops.mlstm_scan(om, rows_m, 0, Hm * 128, 2 * Hm * 128, 2 * Hm * 128 + 2 * Hm * em, 2 * Hm * 128 + 2 * Hm * em + Hm,
-                                     zeros_m, zeros_m, states[i], slots, cu, reqs, Hm, 128, em, 15.0, 128 ** -0.5), sets)
+        row(f"matrix memory{'' if T <= 64 else ' over chunks'}, {Hm} heads of 128 x {em}, {reqs} request(s)", "", T,
+            reqs * 2 * states[0][0].numel() * 4 + T * (wm * 2 + Hm * em * 4),
+            memory_launch((om, rows_m, 0, Hm * 128, 2 * Hm * 128, 2 * Hm * 128 + 2 * Hm * em, 2 * Hm * 128 + 2 * Hm * em + Hm, zeros_m, zeros_m),
+                          states, slots, cu, reqs, T, Hm, 128, em, dev), sets)
         del states
         # the norm over all heads and the gate
         gated = torch.empty(T, H * e, device=dev, dtype=bf)
