@@ -168,8 +168,10 @@ __device__ __forceinline__ void fetch_unit_vectors(float *kt, float *qt, const T
   }
 }
 
+// (up to 16 rows a thread: 64 registers, four blocks to a multiprocessor; left to itself the compiler takes 77 for the bfloat16
+// form, three blocks, and a decode step of 8 requests 7.9 us instead of 6.7)
 template <typename T, int ROWS, int LANES>
-__global__ void __launch_bounds__(SCAN_THREADS)
+__global__ void __launch_bounds__(SCAN_THREADS, ROWS <= 16 ? 4 : 2)
 gated_delta_scan_kernel(float *__restrict__ out, int64_t out_stride, const T *__restrict__ qkv, int64_t qkv_stride, int q_col,
                         int k_col, int v_col, const float *__restrict__ prep, int prep_stride, float *__restrict__ state,
                         int num_state_rows, const int32_t *__restrict__ state_slots, const int32_t *__restrict__ cu_q,
