@@ -6,8 +6,8 @@
 // when temperature < 1e-4 (first maximum), else logits / T, keep values not
 // below the k-th largest, drop the sorted tail whose preceding cumulative
 // probability exceeds top_p, softmax, one multinomial draw from torch's global
-// generator.  Here a cluster of eight blocks handles one row from shared
-// memory, nothing is sorted (the two thresholds are found by radix selection
+// generator.  Here a cluster of blocks handles one row from shared memory or L2,
+// nothing is sorted (the two thresholds are found by radix selection
 // over the ordered bit patterns of the logits: three histogram passes each),
 // the softmax is 32-bit, and the draw is the inverse of the
 // cumulative distribution in token order at a uniform number that depends only
@@ -120,8 +120,8 @@ __global__ void argmax_final_kernel(int32_t *__restrict__ out, const float *__re
 }
 
 // ---- temperature / top-k / top-p sampling.
-// A row belongs to a cluster of SAMPLE_BLOCKS thread blocks; each copies its slice of the row into shared
-// memory once, and every later pass runs from there.  The blocks exchange what they find through distributed
+// A row belongs to a cluster of thread blocks: eight, each with one of the row's SAMPLE_SLICES slices, which it copies into
+// shared memory once and takes every later pass from; or, with many rows, four (WIDE below).  The blocks exchange what they find through distributed
 // shared memory.
 //
 // The two thresholds need no sort.  First by value: bins of equal width below the row's maximum (linear_select), which
@@ -133,7 +133,7 @@ __global__ void argmax_final_kernel(int32_t *__restrict__ out, const float *__re
 // lies in.  Masses are fixed-point integers (2^-40 of the largest probability), so that sums do not depend on
 // the order of the atomic additions.
 namespace cg = cooperative_groups;
-constexpr int SAMPLE_BLOCKS = 8;
+constexpr int SAMPLE_SLICES = 8;           // slices of a row, THREADS runs of consecutive values each: the order of its sums
 constexpr int RADIX_BINS = 2048;
 constexpr float MASS_ONE = 1099511627776.0f;   // 2^40
 
@@ -149,6 +149,7 @@ struct SampleShared {
   unsigned long long warp_mass[33];
   int warp_count[33];
   float warp_f[33];
+  float warp_floor[32];
   int warp_i[33];
   // what block 0 decides for all (read by the others through distributed shared memory)
   int digit;
@@ -168,9 +169,9 @@ struct SampleShared {
   float block_warp_floor;                  // the smallest of the warps' maxima
   int block_odd;                           // a NaN was seen
   int block_argmax;
-  float block_total;
+  float slice_total[2];                    // of the block's slices
   float block_z;
-  int block_last_kept;
+  int slice_last_kept[2];
 };
 
 __device__ __forceinline__ float prob_of(float x, float row_max, float inv_t) { return expf((x - row_max) * inv_t); }
@@ -341,6 +342,53 @@ __device__ uint32_t radix_select(cg::cluster_group &cluster, SampleShared &h, Me
 // the same, or a second level makes bins of their ordered bit patterns, which are even enough within one bin of the first.
 // (With the radix selection behind a list too long, such rows paid for both: one of 128,256 at temperature 2.5 109 us, a
 // flat one 71, where the radix selection alone takes 97 and 43.)  False: the radix selection has to do it.
+//
+// WIDE: a row's cluster is four blocks of 512 threads with two slices each, two blocks to a multiprocessor, and the values
+// stay in L2: some 70 rows run at once where the narrow form (eight blocks of 1,024 threads, slices in shared memory) takes
+// some 16.  With more rows the narrow form's clusters came one after the other, each with its meetings, or two to a
+// multiprocessor with 32 registers a thread: a mixed batch of 64 rows 89 us, now 51.
+constexpr int threads_of(bool wide) { return wide ? THREADS / 2 : THREADS; }
+constexpr int blocks_of(bool wide) { return wide ? SAMPLE_SLICES / 2 : SAMPLE_SLICES; }
+constexpr int WIDE_GROUPS = 4;
+
+// f(index, value, group) for all of a block's values.  WIDE: four of a thread's pieces, of 16 bytes where every group gets
+// some, are asked for at once, and fall into WIDE_GROUPS groups.
+__device__ __forceinline__ bool wide_pieces(const float *vals, int n) {
+  return (reinterpret_cast<uintptr_t>(vals) & 15) == 0 && n >= 4 * WIDE_GROUPS * threads_of(true);
+}
+template <bool WIDE, typename F>
+__device__ __forceinline__ void each_value(const float *vals, int n, F f) {
+  constexpr int T = threads_of(WIDE);
+  if constexpr (!WIDE) {
+    for (int i = threadIdx.x; i < n; i += T) f(i, vals[i], 0);
+  } else if (wide_pieces(vals, n)) {
+    const float4 *src = reinterpret_cast<const float4 *>(vals);
+    const int quads = n / 4;
+    for (int q = threadIdx.x; q < quads; q += WIDE_GROUPS * T) {
+      float4 x[WIDE_GROUPS];
+#pragma unroll
+      for (int j = 0; j < WIDE_GROUPS; ++j)
+        if (q + j * T < quads) x[j] = src[q + j * T];
+#pragma unroll
+      for (int j = 0; j < WIDE_GROUPS; ++j) {
+        const int i = 4 * (q + j * T);
+        if (i < 4 * quads) f(i, x[j].x, j), f(i + 1, x[j].y, j), f(i + 2, x[j].z, j), f(i + 3, x[j].w, j);
+      }
+    }
+    for (int i = quads * 4 + threadIdx.x; i < n; i += T) f(i, vals[i], 0);
+  } else {
+    for (int i = threadIdx.x; i < n; i += WIDE_GROUPS * T) {
+      float x[WIDE_GROUPS];
+#pragma unroll
+      for (int j = 0; j < WIDE_GROUPS; ++j)
+        if (i + j * T < n) x[j] = vals[i + j * T];
+#pragma unroll
+      for (int j = 0; j < WIDE_GROUPS; ++j)
+        if (i + j * T < n) f(i + j * T, x[j], j);
+    }
+  }
+}
+
 constexpr int LIST_MAX = 512;              // (every value of the list meets every other)
 struct BinList {
   unsigned long long mass[LIST_MAX];
@@ -351,33 +399,32 @@ static_assert(sizeof(BinList) <= sizeof(MergedHistogram), "the list lies where t
 // One level: a histogram of the values that take part, its sums over the cluster, the bin in which the sum from `base` on
 // passes the limit (what lies above it: `above`), and that bin's values in block 0's list.  bin_of(x, key): a value's bin,
 // or -1: it takes no part; limit_of(total): the limit.  False: the sum does not pass it.
-template <typename BinOf, typename MassOf, typename LimitOf>
+template <bool WIDE, typename BinOf, typename MassOf, typename LimitOf>
 __device__ __forceinline__ bool select_level(cg::cluster_group &cluster, SampleShared &h, BinList *list, int which, const float *vals,
                                              int n, unsigned long long base, BinOf bin_of, MassOf mass_of, LimitOf limit_of,
                                              int &bin, unsigned long long &above, unsigned long long &limit) {
-  constexpr int SHARE = RADIX_BINS / SAMPLE_BLOCKS;
+  constexpr int BLOCKS = blocks_of(WIDE), SHARE = RADIX_BINS / BLOCKS;
   const int rank = static_cast<int>(cluster.block_rank()), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int b = threadIdx.x; b < RADIX_BINS; b += blockDim.x) h.mass_lo[b] = 0, h.mass_hi[b] = 0;
   if (threadIdx.x == 0) h.listed[which] = 0, h.chosen[which] = 0xffffffffu;
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const float x = vals[i];
+  each_value<WIDE>(vals, n, [&](int, float x, int) {
     const int at = bin_of(x, ordered_key(x));
-    if (at < 0) continue;
+    if (at < 0) return;
     const unsigned long long m = mass_of(x);
-    if (m == 0) continue;
+    if (m == 0) return;
     const unsigned add_lo = static_cast<unsigned>(m), add_hi = static_cast<unsigned>(m >> 32);
     const unsigned old = atomicAdd(&h.mass_lo[at], add_lo);
     const unsigned carry = old + add_lo < old ? 1u : 0u;              // additions with carry commute: the sum is exact
     if (add_hi + carry) atomicAdd(&h.mass_hi[at], add_hi + carry);
-  }
+  });
   cluster.sync();                          // every block's histogram is there
   // this block's share of the bins, summed over the blocks and scanned: warps 0 .. SHARE / 32 - 1, a bin a lane
   unsigned long long mine = 0, upto = 0;
   const int my_bin = rank * SHARE + static_cast<int>(threadIdx.x);
   if (threadIdx.x < SHARE) {
 #pragma unroll
-    for (int other = 0; other < SAMPLE_BLOCKS; ++other) {
+    for (int other = 0; other < BLOCKS; ++other) {
       const SampleShared *theirs = cluster.map_shared_rank(&h, other);
       mine += (static_cast<unsigned long long>(theirs->mass_hi[my_bin]) << 32) + theirs->mass_lo[my_bin];
     }
@@ -396,7 +443,7 @@ __device__ __forceinline__ bool select_level(cg::cluster_group &cluster, SampleS
   }
   cluster.sync();                          // every block's share is summed
   unsigned long long total = 0, before = base;
-  for (int other = 0; other < SAMPLE_BLOCKS; ++other) {
+  for (int other = 0; other < BLOCKS; ++other) {
     if (other == rank) before = base + total;
     total += cluster.map_shared_rank(&h, other)->share[which];
   }
@@ -404,28 +451,43 @@ __device__ __forceinline__ bool select_level(cg::cluster_group &cluster, SampleS
   if (base + total <= limit) return false; // (every block sees the same)
   if (threadIdx.x < SHARE && before + upto - mine <= limit && before + upto > limit) h.bin = my_bin, h.above = before + upto - mine;
   int owner = -1;                          // the last block up to whose share the sum stays within the limit
-  for (unsigned long long sum = base; owner + 1 < SAMPLE_BLOCKS && sum <= limit;) sum += cluster.map_shared_rank(&h, ++owner)->share[which];
+  for (unsigned long long sum = base; owner + 1 < BLOCKS && sum <= limit;) sum += cluster.map_shared_rank(&h, ++owner)->share[which];
   cluster.sync();                          // the owner of that bin has found it
   const SampleShared *from = cluster.map_shared_rank(&h, owner);
   bin = from->bin;
   above = from->above;
   SampleShared *first = cluster.map_shared_rank(&h, 0);
   BinList *all = cluster.map_shared_rank(list, 0);
-  const int rounds = (n + blockDim.x - 1) / blockDim.x;
-  for (int round = 0; round < rounds; ++round) {
-    const int i = round * blockDim.x + threadIdx.x;
-    const float x = i < n ? vals[i] : 0.0f;
-    bool in = i < n && bin_of(x, ordered_key(x)) == bin;
-    unsigned long long m = 0;
-    if (in) m = mass_of(x), in = m != 0;   // (a value without mass is no threshold)
-    const unsigned found = __ballot_sync(0xffffffffu, in);
-    if (found == 0) continue;
-    int at = 0;
-    if (lane == 0) at = atomicAdd(&first->listed[which], __popc(found));
-    at = __shfl_sync(0xffffffffu, at, 0);
-    if (at >= LIST_MAX) break;             // (too many already)
-    at += __popc(found & ((1u << lane) - 1u));
-    if (in && at < LIST_MAX) all->key[at] = ordered_key(x), all->mass[at] = m;
+  if constexpr (WIDE) {
+    bool full = false;                     // (too many already)
+    each_value<WIDE>(vals, n, [&](int, float x, int) {
+      if (full || bin_of(x, ordered_key(x)) != bin) return;
+      const unsigned long long m = mass_of(x);
+      if (m == 0) return;                  // (a value without mass is no threshold)
+      const cg::coalesced_group found = cg::coalesced_threads();
+      int at = 0;
+      if (found.thread_rank() == 0) at = atomicAdd(&first->listed[which], static_cast<int>(found.size()));
+      at = found.shfl(at, 0) + static_cast<int>(found.thread_rank());
+      if (at < LIST_MAX) all->key[at] = ordered_key(x), all->mass[at] = m;
+      else full = true;
+    });
+  } else {
+    const int rounds = (n + blockDim.x - 1) / blockDim.x;
+    for (int round = 0; round < rounds; ++round) {
+      const int i = round * blockDim.x + threadIdx.x;
+      const float x = i < n ? vals[i] : 0.0f;
+      bool in = i < n && bin_of(x, ordered_key(x)) == bin;
+      unsigned long long m = 0;
+      if (in) m = mass_of(x), in = m != 0;   // (a value without mass is no threshold)
+      const unsigned found = __ballot_sync(0xffffffffu, in);
+      if (found == 0) continue;
+      int at = 0;
+      if (lane == 0) at = atomicAdd(&first->listed[which], __popc(found));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (at >= LIST_MAX) break;             // (too many already)
+      at += __popc(found & ((1u << lane) - 1u));
+      if (in && at < LIST_MAX) all->key[at] = ordered_key(x), all->mass[at] = m;
+    }
   }
   cluster.sync();                          // the list is complete
   return true;
@@ -445,6 +507,7 @@ __device__ __forceinline__ uint32_t from_list(cg::cluster_group &cluster, Sample
 }
 
 // Behind a first level whose list was too short for `bin`.
+template <bool WIDE>
 __device__ __noinline__ bool refine_select(SampleShared &h, BinList *list, int which, const float *vals, int n, bool with_mass,
                                            uint32_t min_key, float row_max, float inv_t, float scale, int bin,
                                            unsigned long long above, unsigned long long limit, uint32_t &threshold) {
@@ -455,12 +518,11 @@ __device__ __noinline__ bool refine_select(SampleShared &h, BinList *list, int w
   if (threadIdx.x == 0) h.least = 0xffffffffu, h.most = 0;
   cluster.sync();                          // (and everyone has read the list's length)
   uint32_t lo = 0xffffffffu, hi = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const float x = vals[i];
+  each_value<WIDE>(vals, n, [&](int, float x, int) {
     const uint32_t key = ordered_key(x);
-    if (key < min_key || static_cast<int>(fminf((row_max - x) * scale, static_cast<float>(RADIX_BINS - 1))) != bin || mass_of(x) == 0) continue;
+    if (key < min_key || static_cast<int>(fminf((row_max - x) * scale, static_cast<float>(RADIX_BINS - 1))) != bin || mass_of(x) == 0) return;
     lo = min(lo, key), hi = max(hi, key);
-  }
+  });
   lo = __reduce_min_sync(0xffffffffu, lo), hi = __reduce_max_sync(0xffffffffu, hi);
   if ((threadIdx.x & 31) == 0 && lo <= hi) {
     atomicMin(&first->least, lo);
@@ -475,7 +537,7 @@ __device__ __noinline__ bool refine_select(SampleShared &h, BinList *list, int w
   const int shift = max(0, 21 - __clz(static_cast<int>(hi - lo)));    // (hi - lo) >> shift is below 2,048
   auto bin_of = [&](float, uint32_t key) { return key >= lo && key <= hi ? static_cast<int>((hi - key) >> shift) : -1; };
   const unsigned long long base = above;
-  if (!select_level(cluster, h, list, which, vals, n, base, bin_of, mass_of, [&](unsigned long long) { return limit; }, bin, above, limit))
+  if (!select_level<WIDE>(cluster, h, list, which, vals, n, base, bin_of, mass_of, [&](unsigned long long) { return limit; }, bin, above, limit))
     return false;
   const int listed = first->listed[which];
   if (listed > LIST_MAX) {
@@ -486,6 +548,7 @@ __device__ __noinline__ bool refine_select(SampleShared &h, BinList *list, int w
   return true;
 }
 
+template <bool WIDE>
 __device__ bool linear_select(cg::cluster_group &cluster, SampleShared &h, BinList *list, int which, const float *vals, int n,
                               bool with_mass, int k, float top_p, uint32_t min_key, float row_max, float inv_t, float scale,
                               uint32_t &threshold) {
@@ -498,26 +561,34 @@ __device__ bool linear_select(cg::cluster_group &cluster, SampleShared &h, BinLi
   };
   int bin = 0;
   unsigned long long above = 0, limit = 0;
-  if (!select_level(cluster, h, list, which, vals, n, 0ull, bin_of, mass_of, limit_of, bin, above, limit)) return false;
+  if (!select_level<WIDE>(cluster, h, list, which, vals, n, 0ull, bin_of, mass_of, limit_of, bin, above, limit)) return false;
   const int listed = cluster.map_shared_rank(&h, 0)->listed[which];
-  if (listed > LIST_MAX) return refine_select(h, list, which, vals, n, with_mass, min_key, row_max, inv_t, scale, bin, above, limit, threshold);
+  if (listed > LIST_MAX) return refine_select<WIDE>(h, list, which, vals, n, with_mass, min_key, row_max, inv_t, scale, bin, above, limit, threshold);
   threshold = from_list(cluster, h, list, which, listed, above, limit, min_key);
   return true;
 }
 
-// An inclusive prefix sum over the block's threads in thread order (fixed tree: the same bits every time).
-__device__ float block_inclusive_scan(float v, float *warp_f, float &block_total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (blockDim.x + 31) >> 5;
+// Inclusive prefix sums over a slice's THREADS runs in their order (a fixed tree: the same bits every time, whatever the
+// number of a block's threads): v[h] is the sum of run h * T + threadIdx.x and becomes the sum up to it.
+template <int T>
+__device__ __forceinline__ void slice_inclusive_scan(float (&v)[THREADS / T], float *warp_f, float &slice_total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float up = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += up;
+  for (int h = 0; h < THREADS / T; ++h) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float up = __shfl_up_sync(0xffffffffu, v[h], o);
+      if (lane >= o) v[h] += up;
+    }
   }
   __syncthreads();
-  if (lane == 31) warp_f[warp] = v;
+  if (lane == 31) {
+#pragma unroll
+    for (int h = 0; h < THREADS / T; ++h) warp_f[h * (T / 32) + warp] = v[h];
+  }
   __syncthreads();
   if (warp == 0) {
-    float w = lane < warps ? warp_f[lane] : 0.0f;
+    float w = warp_f[lane];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const float up = __shfl_up_sync(0xffffffffu, w, o);
@@ -526,18 +597,16 @@ __device__ float block_inclusive_scan(float v, float *warp_f, float &block_total
     warp_f[lane] = w;                       // inclusive over warps
   }
   __syncthreads();
-  block_total = warp_f[warps - 1];
-  return v + (warp > 0 ? warp_f[warp - 1] : 0.0f);
+  slice_total = warp_f[THREADS / 32 - 1];
+#pragma unroll
+  for (int h = 0; h < THREADS / T; ++h) v[h] += h * (T / 32) + warp > 0 ? warp_f[h * (T / 32) + warp - 1] : 0.0f;
 }
+static_assert(THREADS == 1024, "one warp adds up the warps' sums");
 
 // params per row: temperature, top_p (floats), top_k, seed_lo, seed_hi, counter (ints).
-// TO_A_SM: blocks a multiprocessor is to hold.  Two (32 registers a thread, some 40 spilled) where there are more blocks
-// than multiprocessors: the waits of one block's meetings are the other's time (64 rows of 128,256 with all kinds of options:
-// 234 us before the selection by value, 107 with it, 96 with two blocks).  One otherwise (a row with top_p 27 us, with
-// 32 registers 31); blocks_to_a_multiprocessor() draws the line.
-// slice: values per block (a multiple of 4); `staged`: the slice fits in shared memory and is copied there.
-template <int TO_A_SM>
-__global__ void __launch_bounds__(THREADS, TO_A_SM)
+// slice: values per slice (a multiple of 4); `staged`: the block's slice fits in shared memory and is copied there (never WIDE).
+template <bool WIDE>
+__global__ void __launch_bounds__(threads_of(WIDE), WIDE ? 2 : 1)
 sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int vocab, int64_t stride, int slice, int staged,
               const float *__restrict__ temperature, const float *__restrict__ top_p, const int32_t *__restrict__ top_k,
               const int32_t *__restrict__ seeds, const float *__restrict__ uniforms, float *__restrict__ probs_out) {
@@ -550,8 +619,9 @@ sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int v
   const int r = blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float *row = logits + r * stride;
-  const int begin = min(vocab, rank * slice);
-  const int n = min(slice, vocab - begin);
+  constexpr int T = threads_of(WIDE), BLOCKS = blocks_of(WIDE), OWN = SAMPLE_SLICES / BLOCKS;   // slices of this block
+  const int begin = min(vocab, rank * OWN * slice);
+  const int n = min(OWN * slice, vocab - begin);
   const float temp = temperature[r];
   const int k = top_k[r];
   const float p_keep = top_p[r];
@@ -577,7 +647,14 @@ sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int v
     float best = -INFINITY;
     int idx = 0x7fffffff;
     bool odd = false;
-    if (filtered) {
+    float group_max[WIDE_GROUPS] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};     // WIDE
+    if constexpr (WIDE) {
+      each_value<WIDE>(vals, n, [&](int i, float x, int group) {
+        odd = odd || x != x;
+        if (x > best || (x == best && begin + i < idx)) { best = x; idx = begin + i; }
+        group_max[group] = fmaxf(group_max[group], x);
+      });
+    } else if (filtered) {
       for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const float x = vals[i];
         if (x != x) odd = true;
@@ -593,6 +670,21 @@ sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int v
     // for a row with filters: the smallest of the threads' maxima (a thread without a value stands aside; NaN: -inf)
     if (filtered) {
       float least = odd ? -INFINITY : (threadIdx.x < n ? best : INFINITY);
+      if constexpr (WIDE) {
+        // (of the groups that have values)
+        const int pieces = wide_pieces(vals, n) ? n / 4 : n;
+        float lowest = INFINITY;
+        least = odd ? -INFINITY : INFINITY;
+#pragma unroll
+        for (int j = 0; j < WIDE_GROUPS; ++j) {
+          if (static_cast<int>(threadIdx.x) + j * T < pieces) least = fminf(least, group_max[j]);
+          float top = group_max[j];
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+          if (warp * 32 + j * T < pieces) lowest = fminf(lowest, top);
+        }
+        if (lane == 0) sh.warp_floor[warp] = lowest;
+      }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
       odd = __any_sync(0xffffffffu, odd);
@@ -618,7 +710,9 @@ sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int v
       }
       if (lane == 0) { sh.block_max = best; sh.block_argmax = idx; }
       if (filtered) {
-        float lowest = lane < warps && lane * 32 < n ? sh.warp_f[lane] : INFINITY;     // (a warp without a value stands aside)
+        float lowest = INFINITY;                                     // (a warp without a value stands aside)
+        if (WIDE && lane < warps) lowest = sh.warp_floor[lane];
+        else if (lane < warps && lane * 32 < n) lowest = sh.warp_f[lane];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) lowest = fminf(lowest, __shfl_xor_sync(0xffffffffu, lowest, o));
         if (lane == 0) sh.block_warp_floor = lowest;
@@ -636,7 +730,7 @@ sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int v
   int best = 0x7fffffff;
   float row_floor = INFINITY, row_warp_floor = INFINITY;
   bool odd = false;
-  for (int other = 0; other < SAMPLE_BLOCKS; ++other) {
+  for (int other = 0; other < BLOCKS; ++other) {
     const SampleShared *theirs = cluster.map_shared_rank(&sh, other);
     const float m = theirs->block_max;
     const int i = theirs->block_argmax;
@@ -667,17 +761,17 @@ sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int v
   };
   const bool plain = !odd && row_max < INFINITY && row_max > -INFINITY;
   if (k > 0 && k < vocab) {
-    // From the maximum down to the smallest of the threads' maxima there are at least as many values as threads that
-    // have one, and down to the smallest of the warps' maxima as many as warps.  Values below take no part: as the last
+    // From the maximum down to the smallest of the threads' maxima there are at least as many values as threads (WIDE:
+    // groups) that have one, and down to the smallest of the warps' maxima as many as warps.  Values below take no part: as the last
     // bin's they were half of a row, added one after the other (top-k 50 of 128,256: 64 rows 99 -> 89 us, 8 rows 26.3 ->
     // 23.7).
-    const int threads = min(vocab, (vocab / slice) * static_cast<int>(blockDim.x));
-    if (slice >= static_cast<int>(blockDim.x) && k <= threads / 32) row_floor = row_warp_floor;
+    const int threads = min(vocab, (vocab / (OWN * slice)) * T * (WIDE ? WIDE_GROUPS : 1));
+    if (k <= threads / 32) row_floor = row_warp_floor;
     const float scale = static_cast<float>(RADIX_BINS - 1) / (row_max - row_floor);
     const uint32_t floor_key = ordered_key(row_floor == 0.0f ? -0.0f : row_floor);     // (0 and -0 are one value here)
     if (plain && k <= threads && row_floor == row_max && row_max != 0.0f) keep_key = ordered_key(row_max);   // k maxima (0: of two signs)
     else if (!(plain && k <= threads && scale > 0.0f && scale < INFINITY &&
-          linear_select(cluster, sh, list, 0, vals, n, false, k, 1.0f, floor_key, row_max, inv_t, scale, keep_key)))
+          linear_select<WIDE>(cluster, sh, list, 0, vals, n, false, k, 1.0f, floor_key, row_max, inv_t, scale, keep_key)))
       keep_key = radix(false, k, 1.0f, 0u);
   }
   if (p_keep < 1.0f) {
@@ -685,52 +779,71 @@ sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int v
     const float scale = static_cast<float>(RADIX_BINS - 1) / 27.8f * inv_t;
     const uint32_t min_key = keep_key;
     if (!(plain && scale < INFINITY &&
-          linear_select(cluster, sh, list, 1, vals, n, true, 0, p_keep, min_key, row_max, inv_t, scale, keep_key)))
+          linear_select<WIDE>(cluster, sh, list, 1, vals, n, true, 0, p_keep, min_key, row_max, inv_t, scale, keep_key)))
       keep_key = radix(true, 0, p_keep, min_key);
   }
 
-  // ---- the kept mass in token order: a thread takes a run of consecutive values of the slice
-  const int chunk = (slice + blockDim.x - 1) / blockDim.x;
-  const int c_begin = min(n, static_cast<int>(threadIdx.x) * chunk), c_end = min(n, c_begin + chunk);
-  float mine = 0.0f;
-  int last_kept = -1;
-  // (runs of whole 16-byte pieces are read as such: single values, a run apart from lane to lane, crowd into few banks)
-  int i0 = c_begin;
-  if (staged && chunk % 4 == 0) {
-    for (; i0 + 4 <= c_end; i0 += 4) {
-      const uint4 four = *reinterpret_cast<const uint4 *>(vals + i0);
-      const uint32_t x[4] = {four.x, four.y, four.z, four.w};
+  // ---- the kept mass in token order: a thread takes runs of consecutive values, THREADS of them to a slice
+  constexpr int RUNS = THREADS / T;
+  const int chunk = (slice + THREADS - 1) / THREADS;
+  const bool pieces = chunk % 4 == 0 && (staged || (reinterpret_cast<uintptr_t>(vals) & 15) == 0);
+  float mine[OWN][RUNS], upto[OWN][RUNS], totals[OWN];
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (ordered_key(x[e]) >= keep_key) { mine += prob_of(__uint_as_float(x[e]), row_max, inv_t); last_kept = begin + i0 + e; }
+  for (int v = 0; v < OWN; ++v) {
+    const int in_slice = max(0, min(slice, n - v * slice));
+    const float *part = vals + v * slice;
+    int last_kept = -1;
+#pragma unroll
+    for (int h = 0; h < RUNS; ++h) {
+      const int c_begin = min(in_slice, (h * T + static_cast<int>(threadIdx.x)) * chunk), c_end = min(in_slice, c_begin + chunk);
+      float sum = 0.0f;
+      // (runs of whole 16-byte pieces are read as such: single values, a run apart from lane to lane, crowd into few banks)
+      int i0 = c_begin;
+      if (pieces) {
+#pragma unroll(WIDE ? 4 : 1)
+        for (; i0 + 4 <= c_end; i0 += 4) {
+          const uint4 four = *reinterpret_cast<const uint4 *>(part + i0);
+          const uint32_t x[4] = {four.x, four.y, four.z, four.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (ordered_key(x[e]) >= keep_key) { sum += prob_of(__uint_as_float(x[e]), row_max, inv_t); last_kept = begin + v * slice + i0 + e; }
+        }
+      }
+      for (int i = i0; i < c_end; ++i)
+        if (ordered_key(part[i]) >= keep_key) { sum += prob_of(part[i], row_max, inv_t); last_kept = begin + v * slice + i; }
+      mine[v][h] = upto[v][h] = sum;
+    }
+    slice_inclusive_scan<T>(upto[v], sh.warp_f, totals[v]);      // mass of the slice's runs up to this one
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) last_kept = max(last_kept, __shfl_xor_sync(0xffffffffu, last_kept, o));
+    if (lane == 0) sh.warp_i[warp] = last_kept;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      sh.slice_total[v] = totals[v];
+      int last = -1;
+      for (int w = 0; w < T / 32; ++w) last = max(last, sh.warp_i[w]);
+      sh.slice_last_kept[v] = last;
+      sh.digit = 0x7fffffff;               // (reused below: the first run past the target)
     }
   }
-  for (int i = i0; i < c_end; ++i)
-    if (ordered_key(vals[i]) >= keep_key) { mine += prob_of(vals[i], row_max, inv_t); last_kept = begin + i; }
-  float mine_total;
-  const float upto_me = block_inclusive_scan(mine, sh.warp_f, mine_total);   // mass of this block's threads 0 .. this one
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) last_kept = max(last_kept, __shfl_xor_sync(0xffffffffu, last_kept, o));
-  if (lane == 0) sh.warp_i[warp] = last_kept;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    sh.block_total = mine_total;
-    int last = -1;
-    for (int w = 0; w < (blockDim.x + 31) >> 5; ++w) last = max(last, sh.warp_i[w]);
-    sh.block_last_kept = last;
-    sh.digit = 0x7fffffff;                 // (reused below: the first thread past the target)
-  }
   cluster.sync();
-  float before = 0.0f, total = 0.0f;       // mass of the blocks before this one, and of all
+  float before[OWN], total = 0.0f;         // mass of the slices before each of this block's, and of all
   int last_of_all = best;
-  bool mass_after_me = false;
-  for (int other = 0; other < SAMPLE_BLOCKS; ++other) {
-    const SampleShared *theirs = cluster.map_shared_rank(&sh, other);
-    const float t = theirs->block_total;
-    if (other == rank) before = total;
-    if (other > rank && t > 0.0f) mass_after_me = true;
+  bool mass_after[OWN];
+#pragma unroll
+  for (int v = 0; v < OWN; ++v) before[v] = 0.0f, mass_after[v] = false;
+#pragma unroll
+  for (int other = 0; other < SAMPLE_SLICES; ++other) {
+    const SampleShared *theirs = cluster.map_shared_rank(&sh, other / OWN);
+    const float t = theirs->slice_total[other % OWN];
+    const int last = theirs->slice_last_kept[other % OWN];
+#pragma unroll
+    for (int v = 0; v < OWN; ++v) {
+      if (other == rank * OWN + v) before[v] = total;
+      if (other > rank * OWN + v && t > 0.0f) mass_after[v] = true;
+    }
     total += t;
-    if (theirs->block_last_kept >= 0) last_of_all = theirs->block_last_kept;
+    if (last >= 0) last_of_all = last;
   }
 
   if (probs_out)
@@ -741,23 +854,34 @@ sample_kernel(int32_t *__restrict__ out, const float *__restrict__ logits, int v
   const uint64_t seed = (static_cast<uint64_t>(static_cast<uint32_t>(seeds[3 * r + 1])) << 32) | static_cast<uint32_t>(seeds[3 * r]);
   const float u = uniforms ? uniforms[r] : uniform_from(seed, static_cast<uint32_t>(seeds[3 * r + 2]));
   const float target = u * total;
-  // the block the target falls into; the last block with mass also takes a target that rounding put past the end
-  const bool here = mine_total > 0.0f && target >= before && (target < before + mine_total || !mass_after_me);
-  if (here) {
-    // the first thread whose running mass passes the target searches its run
-    if (mine > 0.0f && before + upto_me > target) atomicMin(&sh.digit, static_cast<int>(threadIdx.x));
+#pragma unroll
+  for (int v = 0; v < OWN; ++v) {
+    // the slice the target falls into; the last slice with mass also takes a target that rounding put past the end
+    const bool here = totals[v] > 0.0f && target >= before[v] && (target < before[v] + totals[v] || !mass_after[v]);
+    if (!here) continue;                   // (one slice of the row at most, and the whole block agrees)
+    // the first run whose running mass passes the target is searched
+#pragma unroll
+    for (int h = 0; h < RUNS; ++h)
+      if (mine[v][h] > 0.0f && before[v] + upto[v][h] > target) atomicMin(&sh.digit, h * T + static_cast<int>(threadIdx.x));
     __syncthreads();
     const int owner = sh.digit;
     if (owner == 0x7fffffff) {
-      if (threadIdx.x == 0) out[r] = sh.block_last_kept >= 0 ? sh.block_last_kept : last_of_all;
-    } else if (static_cast<int>(threadIdx.x) == owner) {
-      float cum = before + (upto_me - mine);
+      if (threadIdx.x == 0) out[r] = sh.slice_last_kept[v] >= 0 ? sh.slice_last_kept[v] : last_of_all;
+      continue;
+    }
+#pragma unroll
+    for (int h = 0; h < RUNS; ++h) {
+      if (h * T + static_cast<int>(threadIdx.x) != owner) continue;
+      const int in_slice = max(0, min(slice, n - v * slice));
+      const int c_begin = min(in_slice, owner * chunk), c_end = min(in_slice, c_begin + chunk);
+      const float *part = vals + v * slice;
+      float cum = before[v] + (upto[v][h] - mine[v][h]);
       int choice = -1, seen = -1;
       for (int i = c_begin; i < c_end; ++i) {
-        if (ordered_key(vals[i]) < keep_key) continue;
-        seen = begin + i;
-        cum += prob_of(vals[i], row_max, inv_t);
-        if (cum > target) { choice = begin + i; break; }
+        if (ordered_key(part[i]) < keep_key) continue;
+        seen = begin + v * slice + i;
+        cum += prob_of(part[i], row_max, inv_t);
+        if (cum > target) { choice = seen; break; }
       }
       out[r] = choice >= 0 ? choice : seen;
     }
@@ -794,7 +918,7 @@ constexpr size_t MAX_SLICE_BYTES = 152 * 1024;
 // A block's share of a row, whether it is copied into shared memory (where it fits beside the histograms: vocabularies up
 // to about 300,000), and the shared memory that takes.
 size_t slice_smem(int vocab, int &slice, int &staged) {
-  slice = ((vocab + SAMPLE_BLOCKS - 1) / SAMPLE_BLOCKS + 3) / 4 * 4;
+  slice = ((vocab + SAMPLE_SLICES - 1) / SAMPLE_SLICES + 3) / 4 * 4;
   const size_t slice_bytes = static_cast<size_t>(slice) * sizeof(float);
   staged = slice_bytes <= MAX_SLICE_BYTES ? 1 : 0;
   return sizeof(MergedHistogram) + (staged ? slice_bytes : 0);
@@ -803,20 +927,22 @@ size_t slice_smem(int vocab, int &slice, int &staged) {
 // (the same for every vocabulary: another thread's call must not lower it again)
 cudaError_t raise_sample_smem() {
   constexpr int most = static_cast<int>(sizeof(MergedHistogram) + MAX_SLICE_BYTES);
-  cudaError_t e = cudaFuncSetAttribute(sample_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  return e != cudaSuccess ? e : cudaFuncSetAttribute(sample_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  cudaError_t e = cudaFuncSetAttribute(sample_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(sample_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(MergedHistogram));
+  return e;
 }
 
-// Which form a launch takes, asked of the device once per size of shared memory: one block to a multiprocessor where all
-// rows' clusters run at once that way (clusters stay inside one part of the chip: some 16 rows, not 148 / 8), two where two
-// fit (vocabularies up to about 131,000).  128,256 words, rows with top-k, us, one block against two: 16 rows 49 / 43
-// (two waves against one); 151,936 words, where one block fits: 64 rows 140 with 64 registers a thread, 151 with the 32 of
-// the form for two.
-int blocks_to_a_multiprocessor(int num_rows, size_t smem) {
+// Whether a launch takes the wide form, asked of the device once per size of shared memory: where not all rows' clusters
+// of the narrow form run at once (clusters stay inside one part of the chip: some 16 rows, not 148 / 8), for vocabularies
+// up to about 131,000 (two slices to a multiprocessor).  Narrow against wide, us, 128,256 words: 64 rows that are greedy
+// 28.5 / 11.6, at a temperature 49.8 / 24.3, top-p 99 / 51, top-k 89 / 39, both 123 / 56; 40 rows of top-p 77 / 48; 32,000
+// words, 64 rows of top-p 62 / 26.  Larger vocabularies and the rows that run at once stay with the narrow form (8 rows of
+// top-p 27).
+bool takes_wide_form(int num_rows, size_t smem) {
   struct Known {
     int device = -1;
     size_t smem = 0;
-    int rows = 0;                          // that run at once, one block to a multiprocessor
+    int rows = 0;                          // of the narrow form that run at once
     bool two = false;
   };
   thread_local Known known;
@@ -824,22 +950,24 @@ int blocks_to_a_multiprocessor(int num_rows, size_t smem) {
   if (cudaGetDevice(&device) != cudaSuccess) device = 0;
   if (known.device != device || known.smem != smem) {
     cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(SAMPLE_BLOCKS, 1);
+    config.gridDim = dim3(SAMPLE_SLICES, 1);
     config.blockDim = dim3(THREADS);
     config.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = SAMPLE_BLOCKS;
+    attr[0].val.clusterDim.x = SAMPLE_SLICES;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     config.attrs = attr;
     config.numAttrs = 1;
-    int rows = 0, blocks = 0;
-    if (cudaOccupancyMaxActiveClusters(&rows, sample_kernel<1>, &config) != cudaSuccess) rows = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, sample_kernel<2>, THREADS, smem) != cudaSuccess) blocks = 0;
+    int rows = 0, per_sm = 0, reserved = 0;
+    if (cudaOccupancyMaxActiveClusters(&rows, sample_kernel<false>, &config) != cudaSuccess) rows = 0;
+    if (cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device) != cudaSuccess) per_sm = 0;
+    if (cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, device) != cudaSuccess) reserved = 0;
     cudaGetLastError();                    // a refusal is an answer, not an error of the caller
-    known.device = device, known.smem = smem, known.rows = rows, known.two = blocks >= 2;
+    known.device = device, known.smem = smem, known.rows = rows;
+    known.two = 2 * (smem + sizeof(SampleShared) + static_cast<size_t>(reserved)) <= static_cast<size_t>(per_sm);
   }
-  return num_rows > known.rows && known.two ? 2 : 1;
+  return num_rows > known.rows && known.two;
 }
 
 }  // namespace
@@ -848,7 +976,8 @@ int blocks_to_a_multiprocessor(int num_rows, size_t smem) {
 LE_API int le_sample_blocks(int num_rows, int vocab) {
   int slice = 0, staged = 0;
   const size_t smem = slice_smem(vocab, slice, staged);
-  return raise_sample_smem() == cudaSuccess ? blocks_to_a_multiprocessor(num_rows, smem) : 0;
+  if (raise_sample_smem() != cudaSuccess) return 0;
+  return takes_wide_form(num_rows, smem) ? 2 : 1;
 }
 
 // seeds: [rows, 3] = seed low word, seed high word, counter.  `uniforms`
@@ -863,15 +992,17 @@ LE_API int le_sample(int32_t *out, const float *logits, int num_rows, int vocab,
   const size_t smem = slice_smem(vocab, slice, staged);
   if (cudaError_t e = raise_sample_smem(); e != cudaSuccess)
     return le::invalid("le_sample: cannot get %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-  auto *kernel = blocks_to_a_multiprocessor(num_rows, smem) == 2 ? sample_kernel<2> : sample_kernel<1>;
+  const bool wide = takes_wide_form(num_rows, smem);
+  if (wide) staged = 0;
+  auto *kernel = wide ? sample_kernel<true> : sample_kernel<false>;
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(SAMPLE_BLOCKS, num_rows);
-  config.blockDim = dim3(THREADS);
-  config.dynamicSmemBytes = smem;
+  config.gridDim = dim3(blocks_of(wide), num_rows);
+  config.blockDim = dim3(threads_of(wide));
+  config.dynamicSmemBytes = wide ? sizeof(MergedHistogram) : smem;
   config.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = SAMPLE_BLOCKS;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(blocks_of(wide));
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   config.attrs = attr;

@@ -74,3 +74,24 @@ def test_two_blocks_to_a_multiprocessor_only_where_two_fit():
         assert forms[:2] == [1, 1] and forms[-2:] == [2, 2] and forms == sorted(forms)
     for vocab in (151936, 256000, 300000):
         assert [form(n, vocab) for n in (1, 19, 64)] == [1, 1, 1]
+
+
+@pytest.mark.parametrize("vocab", [5, 1023, 8200, 32768, 65537, 128256])
+@pytest.mark.parametrize("kind", ["normal", "masked", "two", "close"])
+def test_a_row_alone_and_among_many(vocab, kind):
+    """Few rows run as clusters of eight blocks, many as clusters of four that hold two slices each: the same tokens and
+    the same probabilities, bit for bit (rows of odd vocabularies start anywhere in a 16-byte piece)."""
+    from lyapunov_engine_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(vocab)
+    n = 39
+    x = rows_of(kind, n, vocab, g)
+    t, p, k = (torch.tensor([OPTIONS[i % len(OPTIONS)][j] for i in range(n)], device=DEV) for j in range(3))
+    t[-1] = 0.0
+    seeds = torch.arange(3 * n, device=DEV, dtype=torch.int32).view(n, 3)
+    out, probs = torch.empty(n, dtype=torch.int32, device=DEV), torch.empty(n, vocab, device=DEV)
+    ops.sample(out, x, t, p, k.int(), seeds, probs_out=probs)
+    assert ops.core().le_sample_blocks(n, vocab) == 2 and ops.core().le_sample_blocks(1, vocab) == 1
+    one, prob = torch.empty(1, dtype=torch.int32, device=DEV), torch.empty(1, vocab, device=DEV)
+    for i in range(n):
+        ops.sample(one, x[i:i + 1], t[i:i + 1], p[i:i + 1], k[i:i + 1].int(), seeds[i:i + 1], probs_out=prob)
+        assert int(one) == int(out[i]) and torch.equal(prob[0], probs[i])
