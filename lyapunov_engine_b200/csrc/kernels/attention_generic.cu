@@ -18,6 +18,11 @@
 // of operations for a token does not depend on which tokens share its tile,
 // so logits are bit-for-bit the same under every cut.
 //
+// What bounds it: shared-memory reads (five of 16 bytes for 16 multiply-adds of a score, two for eight of a value) and a
+// tile's chain of copy, scores, softmax and values; so a thread reads four entries at a time and the next tile's copies
+// (cp.async) run beside a tile's arithmetic.  333 prompt tokens and three decoded ones of 500, 32 heads of 64, float32: 168
+// us with single entries and tiles loaded between two meetings, 95 now, the same bits.
+//
 // Reference: flash_attn_v2_fwd_kernel (csrc/kernels/flash_attn_v2.cu:13-212),
 // whose mask is aligned top-left (key > query index, line 114) and whose keys
 // are contiguous; and paged_attention_kernel (csrc/kernels/paged_attention.cu:9-109).
@@ -34,14 +39,37 @@ constexpr int HD = LE_HEAD_DIM;
 constexpr int QT = 16;   // query rows per block
 constexpr int KT = 32;   // keys per tile
 constexpr int THREADS = 128;
-constexpr int KPAD = HD + 1;
+constexpr int GROUP = HD % 32 == 0 ? 4 : 2;        // neighbouring dimensions of a row's output that a thread owns
 
+// Keys and values lie in their own type, as copied; a key's row is 16 bytes longer than its entries, so that the eight
+// keys that a row's threads read at a time fall into different banks.
+template <typename T>
 struct GenericSmem {
+  static constexpr int KPAD = HD + 16 / static_cast<int>(sizeof(T));
+  static constexpr int STAGE_BYTES = KT * (KPAD + HD) * static_cast<int>(sizeof(T));
+  // the next tile's copies run beside a tile's arithmetic where two tiles leave room for two blocks a multiprocessor
+  static constexpr int STAGES = 2 * STAGE_BYTES + QT * (HD + KT + 4) * 4 <= 100 * 1024 ? 2 : 1;
   float q[QT][HD];
-  float k[KT][KPAD];
-  float v[KT][HD];
-  float s[QT][KT + 1];
+  float s[QT][KT + 4];
+  struct Stage {
+    T k[KT][KPAD];
+    T v[KT][HD];
+  } stage[STAGES];
 };
+
+__device__ __forceinline__ float4 load4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ float4 load4(const __nv_bfloat16 *p) {
+  const uint2 u = *reinterpret_cast<const uint2 *>(p);
+  return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
+                     __uint_as_float(u.y & 0xffff0000u));
+}
+__device__ __forceinline__ float2 load2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
+__device__ __forceinline__ float2 load2(const __nv_bfloat16 *p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(p)); }
+
+__device__ __forceinline__ void copy16(void *smem, const void *gmem, bool valid) {
+  const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(gmem), "r"(valid ? 16 : 0));
+}
 
 template <typename T>
 __global__ void __launch_bounds__(THREADS)
@@ -51,9 +79,11 @@ attention_generic_kernel(T *__restrict__ out, int64_t out_stride, const T *__res
                          const int32_t *__restrict__ ctx_before, const int32_t *__restrict__ tile_request,
                          const int32_t *__restrict__ tile_q0, int num_heads, int num_kv_heads, int page_size,
                          int num_pages, int reach, float scale, const float *__restrict__ head_scale,
-                         int keep_first, float softcap, const float *__restrict__ sink, int *__restrict__ status) {
+                         int keep_first, float softcap, const float *__restrict__ sink, int pieces, int *__restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  GenericSmem &sm = *reinterpret_cast<GenericSmem *>(smem_raw);
+  using Smem = GenericSmem<T>;
+  constexpr int STAGES = Smem::STAGES;
+  Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
 
   const int tile = blockIdx.x, head = blockIdx.y;
   const int kvh = head / (num_heads / num_kv_heads);
@@ -86,43 +116,77 @@ attention_generic_kernel(T *__restrict__ out, int64_t out_stride, const T *__res
   const int keep_tiles = keep_first > 0 ? min((keep_first + KT - 1) / KT, k_begin / KT) : 0;
   const int window_tiles = p_last >= k_begin ? (p_last - k_begin) / KT + 1 : 0;
 
-  for (int it = 0; it < keep_tiles + window_tiles; ++it) {
-    const bool kept_tile = it < keep_tiles;
-    const int k0 = kept_tile ? it * KT : k_begin + (it - keep_tiles) * KT;
-    __syncthreads();
-    // keys and values of this tile, one key row per group of 4 threads
-    {
-      const int kk = tid / 4, part = tid % 4;
-      const int pos = k0 + kk;
-      const bool live = pos <= p_last && (!kept_tile || pos < keep_first);
-      int page = 0;
-      if (live) {
-        page = table[pos / page_size];
-        if (page < 0 || page >= num_pages) {
-          atomicOr(status, LE_STATUS_BAD_PAGE);
-          page = -1;
-        }
-      }
-      const int64_t base = live && page >= 0
-                               ? ((static_cast<int64_t>(page) * num_kv_heads + kvh) * page_size + pos % page_size) * HD
-                               : -1;
-      for (int d = part; d < HD; d += 4) {
-        sm.k[kk][d] = base >= 0 ? le::to_f32(k_cache[base + d]) : 0.0f;
-        sm.v[kk][d] = base >= 0 ? le::to_f32(v_cache[base + d]) : 0.0f;
+  const int tiles = keep_tiles + window_tiles;
+  auto first_key = [&](int it) { return it < keep_tiles ? it * KT : k_begin + (it - keep_tiles) * KT; };
+  // keys and values of a tile, one key row per group of 4 threads
+  auto copy_tile = [&](int it) {
+    typename Smem::Stage &to = sm.stage[it % STAGES];
+    const int kk = tid / 4, part = tid % 4;
+    const int pos = first_key(it) + kk;
+    bool live = pos <= p_last && (it >= keep_tiles || pos < keep_first);
+    int64_t base = 0;
+    if (live) {
+      const int page = table[pos / page_size];
+      if (page < 0 || page >= num_pages) {
+        atomicOr(status, LE_STATUS_BAD_PAGE);
+        live = false;
+      } else {
+        base = ((static_cast<int64_t>(page) * num_kv_heads + kvh) * page_size + pos % page_size) * HD;
       }
     }
-    __syncthreads();
+    constexpr int PER = 16 / static_cast<int>(sizeof(T));
+    if (pieces) {
+#pragma unroll 8
+      for (int d = part * PER; d < HD; d += 4 * PER) {
+        copy16(&to.k[kk][d], k_cache + base + d, live);
+        copy16(&to.v[kk][d], v_cache + base + d, live);
+      }
+    } else {
+      for (int d = part; d < HD; d += 4) {
+        to.k[kk][d] = live ? k_cache[base + d] : le::from_f32<T>(0.0f);
+        to.v[kk][d] = live ? v_cache[base + d] : le::from_f32<T>(0.0f);
+      }
+    }
+  };
+  if (STAGES == 2 && tiles > 0) copy_tile(0);
+  asm volatile("cp.async.commit_group;\n" ::);
+
+  for (int it = 0; it < tiles; ++it) {
+    const int k0 = first_key(it);
+    if constexpr (STAGES == 2) {
+      asm volatile("cp.async.wait_group 0;\n" ::);
+      __syncthreads();                           // tile `it` is there, and everyone is done with the one before
+      if (it + 1 < tiles) copy_tile(it + 1);
+      asm volatile("cp.async.commit_group;\n" ::);
+    } else {
+      __syncthreads();
+      copy_tile(it);
+      asm volatile("cp.async.commit_group;\n" ::);
+      asm volatile("cp.async.wait_group 0;\n" ::);
+      __syncthreads();
+    }
+    const typename Smem::Stage &now = sm.stage[it % STAGES];
 
     // scores of this thread's row against keys sub, sub + 8, sub + 16, sub + 24
     float s[KT / 8];
     float tile_max = -INFINITY;
+    float dots[KT / 8] = {};
+#pragma unroll 4
+    for (int d = 0; d < HD; d += 4) {
+      const float4 x = load4(&sm.q[row][d]);
+#pragma unroll
+      for (int c = 0; c < KT / 8; ++c) {
+        const float4 y = load4(&now.k[sub + 8 * c][d]);
+        dots[c] = fmaf(x.x, y.x, dots[c]);
+        dots[c] = fmaf(x.y, y.y, dots[c]);
+        dots[c] = fmaf(x.z, y.z, dots[c]);
+        dots[c] = fmaf(x.w, y.w, dots[c]);
+      }
+    }
 #pragma unroll
     for (int c = 0; c < KT / 8; ++c) {
-      const int kk = sub + 8 * c;
-      const int pos = k0 + kk;
-      float dot = 0.0f;
-#pragma unroll 8
-      for (int d = 0; d < HD; ++d) dot = fmaf(sm.q[row][d], sm.k[kk][d], dot);
+      const int pos = k0 + sub + 8 * c;
+      const float dot = dots[c];
       const bool seen = row < rows && le::key_visible(pos, p_row, lo_row, keep_first);
       float score = dot * scale;
       if (softcap > 0.0f) score = softcap * tanhf(score / softcap);
@@ -146,13 +210,31 @@ attention_generic_kernel(T *__restrict__ out, int64_t out_stride, const T *__res
     m_run = m_new;
     __syncwarp();  // the 8 threads of a row live in one warp; their probabilities are written
 
-    // weighted values: this thread owns dimensions sub, sub + 8, ...
+    // weighted values: this thread owns GROUP neighbouring dimensions at GROUP * sub, and so on every 8 * GROUP
 #pragma unroll
     for (int j = 0; j < HD / 8; ++j) acc[j] *= alpha;
-    for (int kk = 0; kk < KT; ++kk) {
-      const float p = sm.s[row][kk];
+#pragma unroll(HD <= 128 ? 2 : 1)
+    for (int k4 = 0; k4 < KT; k4 += 4) {
+      const float4 four = load4(&sm.s[row][k4]);
+      const float p[4] = {four.x, four.y, four.z, four.w};
 #pragma unroll
-      for (int j = 0; j < HD / 8; ++j) acc[j] = fmaf(p, sm.v[kk][sub + 8 * j], acc[j]);
+      for (int e = 0; e < 4; ++e) {
+        const T *v = now.v[k4 + e] + GROUP * sub;
+#pragma unroll
+        for (int j = 0; j < HD / 8; j += GROUP) {
+          if constexpr (GROUP == 4) {
+            const float4 x = load4(v + 8 * j);
+            acc[j] = fmaf(p[e], x.x, acc[j]);
+            acc[j + 1] = fmaf(p[e], x.y, acc[j + 1]);
+            acc[j + 2] = fmaf(p[e], x.z, acc[j + 2]);
+            acc[j + 3] = fmaf(p[e], x.w, acc[j + 3]);
+          } else {
+            const float2 x = load2(v + 8 * j);
+            acc[j] = fmaf(p[e], x.x, acc[j]);
+            acc[j + 1] = fmaf(p[e], x.y, acc[j + 1]);
+          }
+        }
+      }
     }
   }
 
@@ -165,7 +247,7 @@ attention_generic_kernel(T *__restrict__ out, int64_t out_stride, const T *__res
     }
     T *o = out + (tok0 + row) * out_stride + head * HD;
 #pragma unroll
-    for (int j = 0; j < HD / 8; ++j) o[sub + 8 * j] = le::from_f32<T>(acc[j] * inv);
+    for (int j = 0; j < HD / 8; ++j) o[GROUP * sub + (j / GROUP) * 8 * GROUP + j % GROUP] = le::from_f32<T>(acc[j] * inv);
   }
 }
 
@@ -191,10 +273,11 @@ LE_API int le_attention_generic(void *out, int64_t out_stride, const void *q, in
   if (num_kv_heads <= 0 || num_heads % num_kv_heads) return le::invalid("le_attention_generic: %d heads do not divide into %d groups", num_heads, num_kv_heads);
   if (num_heads > 65535) return le::invalid("le_attention_generic: too many heads for one launch");
   dim3 grid(num_tiles, num_heads);
-  const size_t smem = sizeof(GenericSmem);
+  const int pieces = ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0;   // (a row is whole ones)
 #define LE_GO(T)                                                                                                       \
   do {                                                                                                                 \
     auto kernel = attention_generic_kernel<T>;                                                                         \
+    const size_t smem = sizeof(GenericSmem<T>);                                                                        \
     if (smem > 48 * 1024) {                                                                                            \
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)); \
       if (e != cudaSuccess) return le::invalid("le_attention_generic: cannot get %zu bytes of shared memory: %s", smem, cudaGetErrorString(e)); \
@@ -203,7 +286,7 @@ LE_API int le_attention_generic(void *out, int64_t out_stride, const void *q, in
                                             static_cast<const T *>(k_cache), static_cast<const T *>(v_cache),          \
                                             block_table, max_blocks, cu_q, ctx_before, tile_request, tile_q0,          \
                                             num_heads, num_kv_heads, page_size, num_pages, reach, scale, head_scale,   \
-                                            keep_first, softcap, sink, status);                                        \
+                                            keep_first, softcap, sink, pieces, status);                                \
   } while (0)
   if (dtype == LE_F32) LE_GO(float);
   else if (dtype == LE_BF16) LE_GO(__nv_bfloat16);
