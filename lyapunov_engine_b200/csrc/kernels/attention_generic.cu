@@ -21,7 +21,7 @@
 // What bounds it: shared-memory reads (five of 16 bytes for 16 multiply-adds of a score, two for eight of a value) and a
 // tile's chain of copy, scores, softmax and values; so a thread reads four entries at a time and the next tile's copies
 // (cp.async) run beside a tile's arithmetic.  333 prompt tokens and three decoded ones of 500, 32 heads of 64, float32: 168
-// us with single entries and tiles loaded between two meetings, 95 now, the same bits.
+// us with single entries and tiles loaded between two meetings, 95 so, 76 with the longest tiles first; the same bits.
 //
 // Reference: flash_attn_v2_fwd_kernel (csrc/kernels/flash_attn_v2.cu:13-212),
 // whose mask is aligned top-left (key > query index, line 114) and whose keys
@@ -85,7 +85,8 @@ attention_generic_kernel(T *__restrict__ out, int64_t out_stride, const T *__res
   constexpr int STAGES = Smem::STAGES;
   Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
 
-  const int tile = blockIdx.x, head = blockIdx.y;
+  // (heads side by side, the list's last tiles first: those of decoded tokens and of a prompt's end, which take longest)
+  const int tile = gridDim.x / num_heads - 1 - blockIdx.x / num_heads, head = blockIdx.x % num_heads;
   const int kvh = head / (num_heads / num_kv_heads);
   const int b = tile_request[tile];
   const int q0 = tile_q0[tile];
@@ -271,8 +272,8 @@ LE_API int le_attention_generic(void *out, int64_t out_stride, const void *q, in
                                 float softcap, const float *sink, int *status, cudaStream_t stream) {
   if (num_tiles <= 0) return 0;
   if (num_kv_heads <= 0 || num_heads % num_kv_heads) return le::invalid("le_attention_generic: %d heads do not divide into %d groups", num_heads, num_kv_heads);
-  if (num_heads > 65535) return le::invalid("le_attention_generic: too many heads for one launch");
-  dim3 grid(num_tiles, num_heads);
+  if (num_heads > 65535 || static_cast<int64_t>(num_tiles) * num_heads > INT32_MAX) return le::invalid("le_attention_generic: too many heads for one launch");
+  dim3 grid(num_tiles * num_heads);
   const int pieces = ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0;   // (a row is whole ones)
 #define LE_GO(T)                                                                                                       \
   do {                                                                                                                 \
