@@ -15,10 +15,11 @@
 // rows lie TY (of A) or 128 / TY (of W) apart, so that the eight threads of a
 // quarter-warp read eight neighbouring rows of W from different banks.
 // What bounds it: many rows, the FMA pipes and next to them the shared-memory
-// reads, RM + RN of 16 bytes per 4 RM RN multiply-adds (336 rows, 16,384 x
-// 2,048: 582 us, 52 % of the pipes' 74 TFLOP/s, against 1,058 in the general
-// form, whose loads of single floats are uncoalesced and whose 4 x 4 outputs a
-// thread need twice the reads); few rows, the bytes of W (4 rows, 128,256 x
+// reads, RM + RN of 16 bytes per 4 RM RN multiply-adds, and their latency where
+// few warps share a scheduler (356 rows, 16,384 x 2,048: 578 us, 56 % of the
+// pipes' 74 TFLOP/s; 512 rows 728 us, 64 %; the general form, whose loads of
+// single floats are uncoalesced and whose 4 x 4 outputs a thread need twice the
+// reads, takes 1,058 for 336 rows); few rows, the bytes of W (4 rows, 128,256 x
 // 2,048: 205 us, 5.1 TB/s, against 1,175), or, where W has few rows, the chain
 // of K dependent multiply-adds (8 rows, 2,048 x 8,192: 62 us, against 635).
 // Tiles turned to [k][row] with pairs of columns in packed multiply-adds were
@@ -102,8 +103,10 @@ struct F32Tile {
   static constexpr size_t SMEM = sizeof(float) * STAGES * STAGE;
 };
 
-template <int TY, int RM, int RN, int KB, int STAGES>
-__global__ void __launch_bounds__(F32_THREADS)
+// QUADS: how many steps of four k stand side by side in the code; a step's reads then run beside the multiply-adds of the
+// one before.  TO_A_SM: blocks to a multiprocessor that the registers are to leave room for (0: as they come).
+template <int TY, int RM, int RN, int KB, int STAGES, int QUADS, int TO_A_SM>
+__global__ void __launch_bounds__(F32_THREADS, TO_A_SM)
 gemm_f32_kernel(float *__restrict__ C, const float *__restrict__ A, const float *__restrict__ W, int M, int N, int K,
                 int64_t lda, int64_t ldw, int64_t ldc) {
   using Tile = F32Tile<TY, RM, RN, KB, STAGES>;
@@ -151,7 +154,7 @@ gemm_f32_kernel(float *__restrict__ C, const float *__restrict__ A, const float 
     asm volatile("cp.async.commit_group;\n" ::);
     const float *as = f32_smem + (kt % STAGES) * Tile::STAGE + ty * PITCH;
     const float *ws = f32_smem + (kt % STAGES) * Tile::STAGE + Tile::A_STAGE + tx * PITCH;
-#pragma unroll(RM *RN >= 32 ? 2 : 4)
+#pragma unroll QUADS
     for (int k = 0; k < KB; k += 4) {
       float4 a[RM], w[RN];
 #pragma unroll
@@ -189,11 +192,11 @@ gemm_f32_kernel(float *__restrict__ C, const float *__restrict__ A, const float 
   }
 }
 
-template <int TY, int RM, int RN, int KB, int STAGES>
+template <int TY, int RM, int RN, int KB, int STAGES, int QUADS = 4, int TO_A_SM = 0>
 int launch_f32(float *C, const float *A, const float *W, int M, int N, int K, int64_t lda, int64_t ldw, int64_t ldc,
                cudaStream_t stream) {
   using Tile = F32Tile<TY, RM, RN, KB, STAGES>;
-  auto kernel = gemm_f32_kernel<TY, RM, RN, KB, STAGES>;
+  auto kernel = gemm_f32_kernel<TY, RM, RN, KB, STAGES, QUADS, TO_A_SM>;
   if (Tile::SMEM > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Tile::SMEM));
     if (e != cudaSuccess) return le::invalid("le_gemm_simt: cannot get %zu bytes of shared memory: %s", Tile::SMEM, cudaGetErrorString(e));
@@ -206,7 +209,10 @@ int launch_f32(float *C, const float *A, const float *W, int M, int N, int K, in
 // The tile shapes, and what a product costs with each: `base` + `per_round` for every round of blocks (one a
 // multiprocessor; blocks beyond the first share its pipes), in microseconds at K = 2,048, of which both are multiples.
 // Fitted to 1 .. 520 rows against 2,048, 3,072, 16,384 and 128,256 columns; the least is within a tenth of the best of
-// 20 shapes measured at all but two of 41 sizes (within a quarter there).
+// 20 shapes measured at all but two of 41 sizes (within a quarter there).  The five largest were measured again with more
+// steps of k side by side (356 and 512 rows, us): 32 x 64, 2,048 x 8,192 436 -> 384; 48 x 64, the same 493 -> 398; 64 x 128
+// with three blocks to a multiprocessor instead of two, 512 rows of 16,384 x 2,048 847 -> 728; 64 x 64 and 64 x 96 are new
+// (356 rows of 16,384 x 2,048: 578, where the best had been 633).
 struct F32Shape {
   int bm, bn;
   float base, per_round;
@@ -216,8 +222,9 @@ constexpr F32Shape F32_SHAPES[] = {
     {4, 64, 18.0f, 13.0f, launch_f32<2, 2, 1, 64, 4>},    {8, 16, 15.0f, 7.0f, launch_f32<8, 1, 1, 64, 8>},
     {8, 32, 15.0f, 9.5f, launch_f32<4, 2, 1, 64, 5>},     {8, 64, 25.0f, 15.0f, launch_f32<2, 4, 1, 32, 4>},
     {16, 16, 12.0f, 10.0f, launch_f32<8, 2, 1, 64, 6>},   {16, 64, 25.0f, 19.5f, launch_f32<4, 4, 2, 32, 4>},
-    {32, 32, 18.0f, 21.0f, launch_f32<8, 4, 2, 32, 4>},   {32, 64, 28.0f, 29.5f, launch_f32<8, 4, 4, 32, 4>},
-    {48, 64, 33.0f, 42.0f, launch_f32<8, 6, 4, 16, 4>},   {64, 128, 48.0f, 100.0f, launch_f32<8, 8, 8, 32, 3>},
+    {32, 32, 18.0f, 21.0f, launch_f32<8, 4, 2, 32, 4>},   {32, 64, 16.0f, 29.8f, launch_f32<8, 4, 4, 32, 3, 8>},
+    {48, 64, 20.0f, 43.4f, launch_f32<8, 6, 4, 32, 3, 8>}, {64, 64, 20.5f, 53.7f, launch_f32<8, 8, 4, 32, 3, 4>},
+    {64, 96, 38.0f, 77.0f, launch_f32<8, 8, 6, 16, 4, 4>}, {64, 128, 38.0f, 97.5f, launch_f32<8, 8, 8, 32, 2, 2, 3>},
 };
 
 const F32Shape *best_shape(int M, int N) {

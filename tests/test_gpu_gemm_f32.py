@@ -19,6 +19,10 @@ DEV = "cuda:0"
     (97, 4100, 44), (200, 9473, 48),                           # 32 x 64
     (110, 3000, 64), (335, 16385, 20),                         # 48 x 64
     (520, 16384, 32), (513, 16385, 12),                        # 64 x 128
+    (384, 3072, 100), (321, 3009, 36),                         # 64 x 64
+    (356, 16384, 28), (321, 16321, 52),                        # 64 x 96
+    (144, 3072, 68), (97, 3011, 132),                          # 48 x 64
+    (128, 2048, 260), (65, 1987, 36),                          # 32 x 64
 ])
 def test_every_tile_shape_gives_the_general_forms_bits(M, N, K):
     from lyapunov_engine_b200 import ops
