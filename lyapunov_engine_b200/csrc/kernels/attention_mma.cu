@@ -437,7 +437,14 @@ constexpr int dc_warp_smem(int tile) { return DC_STAGES * 2 * tile * HD; }   // 
 // written as the split's partial result (or, with one split, as the result).
 // Scratch per (request, head, split): HD floats of unnormalised output, then
 // the maximum (in log2 units) and the sum.
-template <int DC_TILE>
+//
+// BESIDE: the kernel before is the prefill attention of the same step, which lets this one start once the kernel before
+// *it* is complete, the one that wrote the queries and the newest keys; nothing here is that attention's output, so it is
+// waited for by the grid's last block only, at its end, for the kernels behind this one (a block that waits keeps its
+// place on a multiprocessor).  23 requests beside a portion of 777 tokens, 32 heads of 64: the two attentions took 53 us a
+// layer one after the other, 47 side by side.  (An argument instead of a form of its own cost the other steps 30 us of
+// 2,080 at 61 requests.)
+template <int DC_TILE, bool BESIDE>
 __global__ void __launch_bounds__(DC_THREADS)
 attention_decode_kernel(bf16 *__restrict__ out, int64_t out_stride, float *__restrict__ part_o, float *__restrict__ part_ml,
                         const bf16 *__restrict__ q, int64_t q_stride, const bf16 *__restrict__ k_cache,
@@ -464,12 +471,14 @@ attention_decode_kernel(bf16 *__restrict__ out, int64_t out_stride, float *__res
   const KvLayout kv = make_kv_layout(k_cache, v_cache, block_table + static_cast<int64_t>(b) * max_blocks, kvh,
                                      num_kv_heads, page_size, page_shift, num_pages);
 
+  const bool last_block = blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1 && blockIdx.z == gridDim.z - 1;
   // A request at position 0 whose first page is the page that nobody owns is padding of a step of fixed shape (a
   // real request's first token has a page of its own).  Its row is left zero and the block ends at once, and with
   // it its whole cluster, which is that request's: such blocks then pass through the multiprocessors beside the
   // real ones without holding a place for longer than their launch.
   if (p == 0 && kv.table[0] == num_pages - 1) {
     const int64_t first = (static_cast<int64_t>(blockIdx.z) * num_heads + h0) * num_splits + split;
+    if (BESIDE && last_block) le::wait_for_predecessor();
     for (int i = tid; i < heads_here * HD; i += DC_THREADS) {
       const int row = i / HD, d = i % HD;
       if (num_splits == 1 || cluster_merge) {
@@ -520,7 +529,7 @@ attention_decode_kernel(bf16 *__restrict__ out, int64_t out_stride, float *__res
   };
   // The first tiles are asked for while the kernel before this one still runs, unless they hold the key at
   // position p, which that kernel writes.
-  auto older_than_this_step = [&](int i) { return position_of(tile_start(i)) + DC_TILE <= p; };
+  auto older_than_this_step = [&](int i) { return BESIDE || position_of(tile_start(i)) + DC_TILE <= p; };
   bool late = false;
 #pragma unroll
   for (int s = 0; s < DC_STAGES - 1; ++s) {
@@ -530,7 +539,7 @@ attention_decode_kernel(bf16 *__restrict__ out, int64_t out_stride, float *__res
     }
     cp_async_commit();
   }
-  le::wait_for_predecessor();
+  if (!BESIDE) le::wait_for_predecessor();
   if (late) {                                 // (only the warps at the very end of a request's keys)
 #pragma unroll
     for (int s = 0; s < DC_STAGES - 1; ++s)
@@ -547,7 +556,8 @@ attention_decode_kernel(bf16 *__restrict__ out, int64_t out_stride, float *__res
     for (int i = 0; i < 4; ++i) {
       const int row = g + (i & 1) * 8;
       const int dim = ks * 16 + 2 * t + (i >> 1) * 8;
-      qf[ks][i] = row < heads_here ? *reinterpret_cast<const uint32_t *>(q + tok * q_stride + (h0 + row) * HD + dim) : 0u;
+      const uint32_t *pair = reinterpret_cast<const uint32_t *>(q + tok * q_stride + (h0 + row) * HD + dim);
+      qf[ks][i] = row < heads_here ? (BESIDE ? __ldcg(pair) : *pair) : 0u;
     }
   }
 
@@ -737,6 +747,7 @@ attention_decode_kernel(bf16 *__restrict__ out, int64_t out_stride, float *__res
     }
     le::cluster_sync();                       // nobody leaves while another still reads its shared memory
   }
+  if (BESIDE && last_block) le::wait_for_predecessor();
 }
 
 // out[request, head] = sum_s 2^(m_s - m) O_s / sum_s 2^(m_s - m) l_s
@@ -866,8 +877,10 @@ struct DecodeForm {
   // the kernel may ask for its shared memory (done once)
   static bool ready() {
     static const bool ok = smem() <= 48 * 1024 ||
-                           cudaFuncSetAttribute(attention_decode_kernel<TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                static_cast<int>(smem())) == cudaSuccess;
+                           (cudaFuncSetAttribute(attention_decode_kernel<TILE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 static_cast<int>(smem())) == cudaSuccess &&
+                            cudaFuncSetAttribute(attention_decode_kernel<TILE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 static_cast<int>(smem())) == cudaSuccess);
     if (!ok) cudaGetLastError();
     return ok;
   }
@@ -884,7 +897,7 @@ struct DecodeForm {
     config.attrs = attr;
     config.numAttrs = 1;
     int clusters = 0;
-    const bool ok = cudaOccupancyMaxActiveClusters(&clusters, attention_decode_kernel<TILE>, &config) == cudaSuccess;
+    const bool ok = cudaOccupancyMaxActiveClusters(&clusters, attention_decode_kernel<TILE, false>, &config) == cudaSuccess;
     cudaGetLastError();                                    // a refusal is an answer, not an error of the caller
     return ok && clusters > 0 ? clusters : 0;
   }
@@ -901,7 +914,8 @@ struct DecodeForm {
     if (known[num_splits] == 0) {
       bool fits = true;
       if (num_splits > 8)
-        fits = cudaFuncSetAttribute(attention_decode_kernel<TILE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        fits = cudaFuncSetAttribute(attention_decode_kernel<TILE, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+               cudaFuncSetAttribute(attention_decode_kernel<TILE, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
       const int clusters = fits ? clusters_resident(num_splits) : 0;
       cudaGetLastError();                                  // a refusal above is an answer, not an error of the caller
       known[num_splits] = clusters > 0 ? clusters : -1;
@@ -918,7 +932,7 @@ struct DecodeForm {
     static const int64_t single = [] {
       int device = 0, sms = 0, per_sm = 0;
       if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attention_decode_kernel<TILE>, DC_THREADS, smem()) != cudaSuccess) {
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attention_decode_kernel<TILE, false>, DC_THREADS, smem()) != cudaSuccess) {
         cudaGetLastError();
         return int64_t{0};
       }
@@ -930,11 +944,12 @@ struct DecodeForm {
                     const void *k_cache, const void *v_cache, const int32_t *block_table, int max_blocks, const int32_t *cu_q,
                     const int32_t *ctx_before, const int32_t *requests, int num_requests, int num_heads, int num_kv_heads,
                     int page_size, int num_pages, int reach, float scale, const float *head_scale, int keep_first, float softcap,
-                    const float *sink, int num_splits, int *status) {
+                    const float *sink, int num_splits, int beside, int *status) {
     if (!ready()) return le::invalid("le_attention_decode_bf16: cannot get %zu bytes of shared memory", smem());
+    const auto kernel = beside ? attention_decode_kernel<TILE, true> : attention_decode_kernel<TILE, false>;
     if (cluster_fits(num_splits)) {
       // the splits of a (request, kv head) as one cluster: merged through shared memory, no scratch, no second kernel
-      return le::launch_chained_cluster(attention_decode_kernel<TILE>, grid, dim3(DC_THREADS), smem(), stream, num_splits,
+      return le::launch_chained_cluster(kernel, grid, dim3(DC_THREADS), smem(), stream, num_splits,
                                         static_cast<bf16 *>(out), out_stride, static_cast<float *>(nullptr),
                                         static_cast<float *>(nullptr), static_cast<const bf16 *>(q), q_stride,
                                         static_cast<const bf16 *>(k_cache), static_cast<const bf16 *>(v_cache), block_table,
@@ -946,7 +961,7 @@ struct DecodeForm {
     if (reinterpret_cast<uintptr_t>(scratch) % 8) return le::invalid("le_attention_decode_bf16: the scratch memory must start on an 8-byte boundary");
     float *part_o = scratch;
     float *part_ml = scratch ? scratch + static_cast<int64_t>(num_requests) * num_heads * num_splits * HD : nullptr;
-    int rc = le::launch_chained(attention_decode_kernel<TILE>, grid, dim3(DC_THREADS), smem(), stream, static_cast<bf16 *>(out), out_stride,
+    int rc = le::launch_chained(kernel, grid, dim3(DC_THREADS), smem(), stream, static_cast<bf16 *>(out), out_stride,
                                 part_o, part_ml, static_cast<const bf16 *>(q), q_stride, static_cast<const bf16 *>(k_cache),
                                 static_cast<const bf16 *>(v_cache), block_table, max_blocks, cu_q, ctx_before, requests, num_heads,
                                 num_kv_heads, page_size, page_shift_of(page_size), num_pages, reach, scale, head_scale, keep_first,
@@ -991,6 +1006,9 @@ LE_API int le_attention_decode_resident_blocks(int num_splits, int small) {
 // `form`: 0 lets the number of blocks decide between the usual form of the kernel and the one with 16-key tiles
 // (see small_form); 1 asks for the usual form, 2 for the small one where the head size has it (a caller that pads
 // the step with dummy requests knows how many of the blocks are real; the grid does not show it).
+// With LE_DECODE_BESIDE added the launch before it on the stream must be le_attention_prefill_tc_bf16_before_decode for
+// other requests of the same step: the two then run side by side.
+constexpr int LE_DECODE_BESIDE = 4;
 LE_API int le_attention_decode_bf16_form(void *out, int64_t out_stride, float *scratch, const void *q, int64_t q_stride,
                                          const void *k_cache, const void *v_cache, const int32_t *block_table, int max_blocks,
                                          const int32_t *cu_q, const int32_t *ctx_before, const int32_t *requests,
@@ -1004,16 +1022,18 @@ LE_API int le_attention_decode_bf16_form(void *out, int64_t out_stride, float *s
   const int row_tiles = (group + 15) / 16;
   if (num_kv_heads * row_tiles > 65535 || num_requests > 65535) return le::invalid("le_attention_decode_bf16: the batch is too large for one launch");
   dim3 grid(num_splits, num_kv_heads * row_tiles, num_requests);
+  const int beside = (form & LE_DECODE_BESIDE) != 0 ? 1 : 0;
+  form &= ~LE_DECODE_BESIDE;
   const bool small = form == 0 ? small_form(static_cast<int64_t>(grid.y) * grid.z)
                                : (form == 2 && DC_TILE_DEFAULT == 32 && small_tiles_enabled() && DecodeForm<16>::ready());
   if (small)
     return DecodeForm<16>::launch(grid, stream, out, out_stride, scratch, q, q_stride, k_cache, v_cache, block_table, max_blocks, cu_q,
                                   ctx_before, requests, num_requests, num_heads, num_kv_heads, page_size, num_pages, reach, scale,
-                                  head_scale, keep_first, softcap, sink, num_splits, status);
+                                  head_scale, keep_first, softcap, sink, num_splits, beside, status);
   return DecodeForm<DC_TILE_DEFAULT>::launch(grid, stream, out, out_stride, scratch, q, q_stride, k_cache, v_cache, block_table,
                                              max_blocks, cu_q, ctx_before, requests, num_requests, num_heads, num_kv_heads, page_size,
                                              num_pages, reach, scale, head_scale, keep_first, softcap, sink, num_splits,
-                                             status);
+                                             beside, status);
 }
 
 LE_API int le_attention_decode_bf16(void *out, int64_t out_stride, float *scratch, const void *q, int64_t q_stride,

@@ -95,7 +95,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     const int32_t *__restrict__ ctx_before, const int32_t *__restrict__ tile_request,
                     const int32_t *__restrict__ tile_q0, int num_heads, int num_kv_heads, int page_size, int page_shift,
                     int num_pages, int reach, float scale, const float *__restrict__ head_scale,
-                    const float *__restrict__ sink, int *__restrict__ status) {
+                    const float *__restrict__ sink, int before_decode, int *__restrict__ status) {
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~uintptr_t(1023));
   unsigned char *q_smem = smem;                // [2 heads]
@@ -183,6 +183,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // up to here the block overlapped that kernel's end; nothing of its output is read before this line, and
     // every other role works on what this warp's copies bring.
     le::wait_for_predecessor();
+    // The decode attention of the same step may start here: it needs what this kernel needs, which is complete, and
+    // waits for this kernel's end at its own end only (attention_mma.cu).
+    if (before_decode) le::let_successor_start();
     // The first copies need nothing but the barriers: they start before tensor memory is set up and the block
     // meets, so the scores of tile 0 can follow the block's start closely.
     if (lane == 0) {
@@ -446,6 +449,14 @@ LE_API int le_attention_tc_available(int page_size) {
   return shift >= 3 && page_size <= 128 ? 1 : 0;
 }
 
+// before_decode: the launch that follows on the stream is a decode attention with `beside` set.
+static int launch_prefill_tc(void *out, int64_t out_stride, const void *q, int64_t q_stride, int num_tokens, int q_width,
+                             const void *k_cache, const void *v_cache, const int32_t *block_table, int max_blocks,
+                             const int32_t *cu_q, const int32_t *ctx_before, const int32_t *tile_request,
+                             const int32_t *tile_q0, int num_tiles, int num_heads, int num_kv_heads, int page_size,
+                             int num_pages, int reach, float scale, const float *head_scale, const float *sink,
+                             int before_decode, int *status, cudaStream_t stream);
+
 // Same arguments as le_attention_prefill_bf16 plus the shape of the buffer q
 // lives in; the tiles list 128 query tokens each.  q must be 16-byte aligned
 // with q_stride a multiple of 8; out rows must be 16-byte aligned.
@@ -456,6 +467,32 @@ LE_API int le_attention_prefill_tc_bf16(void *out, int64_t out_stride, const voi
                                         int num_kv_heads, int page_size, int num_pages, int reach, float scale, const float *head_scale,
                                         const float *sink, int *status,
                                         cudaStream_t stream) {
+  return launch_prefill_tc(out, out_stride, q, q_stride, num_tokens, q_width, k_cache, v_cache, block_table, max_blocks, cu_q, ctx_before,
+                           tile_request, tile_q0, num_tiles, num_heads, num_kv_heads, page_size, num_pages, reach, scale, head_scale,
+                           sink, 0, status, stream);
+}
+
+// The same for a step whose decode attention follows at once (le_attention_decode_bf16_form with LE_DECODE_BESIDE) and
+// runs beside this kernel: 112 blocks of a portion of 777 tokens leave 36 multiprocessors without work.
+LE_API int le_attention_prefill_tc_bf16_before_decode(void *out, int64_t out_stride, const void *q, int64_t q_stride, int num_tokens,
+                                                      int q_width, const void *k_cache, const void *v_cache,
+                                                      const int32_t *block_table, int max_blocks, const int32_t *cu_q,
+                                                      const int32_t *ctx_before, const int32_t *tile_request,
+                                                      const int32_t *tile_q0, int num_tiles, int num_heads, int num_kv_heads,
+                                                      int page_size, int num_pages, int reach, float scale,
+                                                      const float *head_scale, const float *sink, int *status,
+                                                      cudaStream_t stream) {
+  return launch_prefill_tc(out, out_stride, q, q_stride, num_tokens, q_width, k_cache, v_cache, block_table, max_blocks, cu_q, ctx_before,
+                           tile_request, tile_q0, num_tiles, num_heads, num_kv_heads, page_size, num_pages, reach, scale, head_scale,
+                           sink, 1, status, stream);
+}
+
+static int launch_prefill_tc(void *out, int64_t out_stride, const void *q, int64_t q_stride, int num_tokens, int q_width,
+                             const void *k_cache, const void *v_cache, const int32_t *block_table, int max_blocks,
+                             const int32_t *cu_q, const int32_t *ctx_before, const int32_t *tile_request,
+                             const int32_t *tile_q0, int num_tiles, int num_heads, int num_kv_heads, int page_size,
+                             int num_pages, int reach, float scale, const float *head_scale, const float *sink,
+                             int before_decode, int *status, cudaStream_t stream) {
   if (num_tiles <= 0) return 0;
   if (!le_attention_tc_available(page_size)) return le::invalid("le_attention_prefill_tc_bf16: pages of %d keys are not supported (8..128, a power of two)", page_size);
   if (num_kv_heads <= 0 || num_heads % num_kv_heads) return le::invalid("le_attention_prefill_tc_bf16: %d heads do not divide into %d groups", num_heads, num_kv_heads);
@@ -478,7 +515,8 @@ LE_API int le_attention_prefill_tc_bf16(void *out, int64_t out_stride, const voi
   dim3 grid(num_kv_heads * ((group + 1) / 2), num_tiles);   // two heads of a group per block
   return le::launch_chained(attention_tc_kernel, grid, dim3(THREADS), smem, stream, map_q, map_k, map_v, static_cast<bf16 *>(out),
                             out_stride, block_table, max_blocks, cu_q, ctx_before, tile_request, tile_q0, num_heads,
-                            num_kv_heads, page_size, tc_page_shift_of(page_size), num_pages, reach, scale, head_scale, sink, status);
+                            num_kv_heads, page_size, tc_page_shift_of(page_size), num_pages, reach, scale, head_scale, sink,
+                            before_decode, status);
 }
 
 #else

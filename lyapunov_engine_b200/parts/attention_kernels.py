@@ -150,12 +150,14 @@ def run(out, qkv, ctx, kv, num_heads, num_kv_heads, head_dim, reach, scale, head
     window = reach
     if out.dtype == torch.bfloat16 and ops.attention_mma_available(head_dim):
         req, q0, n_tiles, n_multi = ctx.tiles[PREFILL_TILE]
+        beside = False          # the decode kernel runs beside the prompt portions' kernel
         if n_multi:
             if (USE_TC_ATTENTION and head_scale_positive and not keep_first and not softcap
                     and ops.attention_tc_available(head_dim, kv.page_size)):
+                beside = ctx.num_decode > 0
                 ops.attention_prefill_tc_bf16(out, qkv, qkv.stride(0), kv.k, kv.v, table, ctx.cu_q, ctx.ctx_before, req, q0,
                                               n_multi, num_heads, num_kv_heads, head_dim, kv.page_size, window, scale,
-                                              ctx.status, head_scale=head_scale, sink=sink)
+                                              ctx.status, head_scale=head_scale, sink=sink, before_decode=beside)
             else:
                 ops.attention_prefill_bf16(out, qkv, qkv.stride(0), kv.k, kv.v, table, ctx.cu_q, ctx.ctx_before, req, q0,
                                            n_multi, num_heads, num_kv_heads, head_dim, kv.page_size, window, scale,
@@ -172,7 +174,7 @@ def run(out, qkv, ctx, kv, num_heads, num_kv_heads, head_dim, reach, scale, head
             ops.attention_decode_bf16(out, scratch, qkv, qkv.stride(0), kv.k, kv.v, table, ctx.cu_q, ctx.ctx_before,
                                       requests, ctx.num_decode, num_heads, num_kv_heads, head_dim, kv.page_size,
                                       window, scale, splits, ctx.status, small_form=small, head_scale=head_scale,
-                                      keep_first=keep_first, softcap=softcap, sink=sink)
+                                      keep_first=keep_first, softcap=softcap, sink=sink, beside=beside)
         return
     req, q0, n_tiles, _ = ctx.tiles[GENERIC_TILE]
     ops.attention_generic(out, qkv, qkv.stride(0), kv.k, kv.v, table, ctx.cu_q, ctx.ctx_before, req, q0, n_tiles,

@@ -149,6 +149,38 @@ def test_tensor_core_kernels(case):
         torch.testing.assert_close(out.float().cpu(), c["want"], atol=2e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("splits", [1, 3, 20])
+@pytest.mark.parametrize("case", [
+    (8, 2, 64, 16, [300, 1, 1, 129, 1], [0, 50, 0, 1000, 4095], None),
+    (24, 8, 128, 16, [1, 200, 1], [900, 700, 31], None),
+    (32, 8, 64, 16, [1500] + [1] * 40, [700] + [97 * i for i in range(40)], 160),
+])
+def test_decode_beside_prompt_portions(case, splits):
+    """The decode kernel started beside the portions' kernel writes the bits that it writes behind it, and what follows
+    on the stream sees both kernels' rows."""
+    from lyapunov_engine_b200 import ops
+    nh, nkv, hd, page, q_lens, ctx_before, window = case
+    c = build_case(torch.bfloat16, nh, nkv, hd, page, q_lens, ctx_before, seed=hd + len(q_lens), window=window)
+    status = ops.new_status(DEV)
+    tiles = [(b, s) for b, n in enumerate(q_lens) if n > 1 for s in range(0, n, 128)]
+    req, q0 = (torch.tensor([t[i] for t in tiles], dtype=torch.int32, device=DEV) for i in range(2))
+    single = torch.tensor([b for b, n in enumerate(q_lens) if n == 1], dtype=torch.int32, device=DEV)
+    scratch = torch.full((max(ops.attention_decode_scratch_floats(hd, len(single), nh, splits), 1),), float("nan"), device=DEV)
+    outs = []
+    for beside in (False, True, True, True):
+        q = torch.zeros_like(c["q"])
+        out = torch.full((c["T"], nh * hd), 7.0, dtype=torch.bfloat16, device=DEV)
+        q.copy_(c["q"])                           # (what both kernels read is written just before them)
+        ops.attention_prefill_tc_bf16(out, q, q.stride(0), c["k"], c["v"], c["table"], c["cu"], c["ctx"], req, q0, len(tiles),
+                                      nh, nkv, hd, page, window, 1.0 / hd ** 0.5, status, before_decode=beside)
+        ops.attention_decode_bf16(out, scratch, q, q.stride(0), c["k"], c["v"], c["table"], c["cu"], c["ctx"], single,
+                                  len(single), nh, nkv, hd, page, window, 1.0 / hd ** 0.5, splits, status, beside=beside)
+        outs.append(out.clone())
+    ops.check_status(status)
+    torch.testing.assert_close(outs[0].float().cpu(), c["want"], atol=2e-2, rtol=2e-2)
+    assert all(torch.equal(o, outs[0]) for o in outs[1:])
+
+
 def test_decode_splits_choice():
     """On this device: no choice puts more blocks into a wave than the device
     holds, one split where the batch fills the device by itself, and never
